@@ -173,7 +173,8 @@ int qbc_index_build_device(const qbc_graph *g, int kind, const int32_t *node_ord
     const qbc::TailEngine tail = [device](qbc::DenseTail &dt) { qbc::device_dense_eliminate(device, dt); };
     p->h.host = qbc::prepare_index(g->g, kind == QBC_INDEX_MHL ? qbc::IndexKind::MHL : qbc::IndexKind::H2H,
                                    node_order ? &o : nullptr, seps, dense_tail_size(g->g.n), tail);
-    qbc::device_build(p->h, device, seps);
+    p->h.host.seps = std::move(seps);
+    qbc::device_build(p->h, device);
     *out = p.release();
   });
 }

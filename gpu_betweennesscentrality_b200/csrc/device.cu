@@ -47,6 +47,7 @@ constexpr unsigned kFull = 0xffffffffu;
 
 // ------------------------------------------------------------------------------- K1 + K2
 struct LabelArgs {
+  const int32_t *guard;  // null, or the kernel leaves at once while *guard is 0
   // label distances, shifted left by `bits` when the packed-key kernel applies (one array serves
   // both kernels: the general one shifts back as it loads)
   const int32_t *__restrict__ dis;
@@ -87,6 +88,7 @@ __device__ __forceinline__ int lca_depth(const int32_t *lo, const int32_t *hi, i
 
 template <int K, bool COUNTS>
 __global__ void __launch_bounds__(256, 1) k_label_scan(LabelArgs a) {
+  if (a.guard && __ldcg(a.guard) == 0) return;
   constexpr int G = 32 / K;
   extern __shared__ int4 smem4[];
   int32_t *sm = reinterpret_cast<int32_t *>(smem4);
@@ -308,6 +310,7 @@ __host__ __device__ constexpr size_t packed_smem(int warps, int S) {
 // entries j >= S of a scan (taller trees) are read from global memory, 4 at a time.
 template <bool COUNTS, int WARPS, bool MP>
 __global__ void __launch_bounds__(WARPS * 32, 1) k_label_scan_packed(LabelArgs a) {
+  if (a.guard && __ldcg(a.guard) == 0) return;
   constexpr int G = 32;
   extern __shared__ int4 smem4[];
   uint32_t *s_key = reinterpret_cast<uint32_t *>(smem4);
@@ -617,6 +620,7 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 
 template <bool COUNTS, int WARPS, int RING>
 __global__ void __launch_bounds__(WARPS * 32, 1) k_label_scan_tall(LabelArgs a) {
+  if (a.guard && __ldcg(a.guard) == 0) return;
   constexpr int G = kTallSources;
   extern __shared__ int4 smem4[];
   uint32_t *s_key = reinterpret_cast<uint32_t *>(smem4);
@@ -842,6 +846,7 @@ __host__ __device__ constexpr size_t rows16_smem(int warps, int S, int R) {
 
 template <bool COUNTS, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, 1) k_label_scan_rows16(LabelArgs a) {
+  if (a.guard && __ldcg(a.guard) == 0) return;
   constexpr int G = kTallSources;
   extern __shared__ int4 smem4[];
   uint32_t *s_key = reinterpret_cast<uint32_t *>(smem4);
@@ -1157,6 +1162,7 @@ __device__ __forceinline__ void finish_pair(const LabelArgs &a, bool have, int k
 
 template <bool COUNTS>
 __global__ void __launch_bounds__(kPairWarps * 32, 1) k_label_scan_pair(LabelArgs a) {
+  if (a.guard && __ldcg(a.guard) == 0) return;
   constexpr int G = 32;
   extern __shared__ int4 smem4[];
   uint32_t *s_key = reinterpret_cast<uint32_t *>(smem4);
@@ -1395,6 +1401,7 @@ struct DepArgs {
   int32_t *lcnt;   // [ns][2*(n_pad+2)] global layer counters when shared ones do not suffice
   double *bc;      // [n] tid order, FP64 red target
   int32_t *err;
+  const int32_t *guard;  // null, or the pass is left out while *guard is 0
 };
 // The label-free sweep's records carry DAG-successor masks in their last word until rho overwrites
 // it (bit k for the k-th of the first four arcs, bit 4 for a later arc); k_dependency_cta_pipe<true>
@@ -1474,7 +1481,9 @@ __device__ __forceinline__ void set_rho(int4 *r, double x) { reinterpret_cast<do
 // A dependency pass leaves at once when the error word is set: the rows it would read come from a
 // label scan or sweep that gave up (its hop layers could index past the layer counters), and the
 // call reports the error anyway.
-__device__ __forceinline__ bool rows_failed(const DepArgs &a) { return a.err && __ldcg(a.err) != ERR_NONE; }
+__device__ __forceinline__ bool rows_failed(const DepArgs &a) {
+  return (a.err && __ldcg(a.err) != ERR_NONE) || (a.guard && __ldcg(a.guard) == 0);
+}
 
 // delta of v, its rho stored in its record, 0.5 * delta added into BC
 template <class RV>
@@ -2267,7 +2276,7 @@ static uint32_t row_wait_spins() {
 // need_hop false: the caller's next kernel does not read the hop rows (label-free index with the
 // CTA pipelined dependency pass, which walks the sweep's wave queue), so the sweep leaves them out.
 static void launch_label(const Handle &h, DeviceState *d, int buf, const int32_t *src, int32_t ns, bool plain,
-                         cudaStream_t st, bool need_hop = true) {
+                         cudaStream_t st, bool need_hop = true, const int32_t *guard = nullptr) {
   if (h.host.kind == IndexKind::CSR) {  // no labels: shortest-path sweeps give the rows
     std::pair<cudaEvent_t, cudaEvent_t> ev{};
     if (d->profiling) {
@@ -2307,6 +2316,7 @@ static void launch_label(const Handle &h, DeviceState *d, int buf, const int32_t
   a.bits = d->packed_bits;
   a.err = d->err;
   a.wait_spins = row_wait_spins();
+  a.guard = guard;
   const int groups = (ns + p.G - 1) / p.G;
   CK(cudaMemsetAsync(d->maxhop[buf], 0, (size_t)ns * 4, st));
   k_src_rows<<<(ns + 127) / 128, 128, 0, st>>>(src, ns, d->depth, d->parent, d->send, d->hmax_pad, d->src_rows[buf]);
@@ -2354,8 +2364,9 @@ static DepArgs dep_args(DeviceState *d, int buf, const int32_t *src, int32_t ns)
 // plain = a single source: one CTA runs its dependency pass (the warp form would leave 7/8 of the
 // CTA idle)
 static void launch_dep(const Handle &h, DeviceState *d, int buf, const int32_t *src, int32_t ns, cudaStream_t st,
-                       bool plain = false) {
+                       bool plain = false, const int32_t *guard = nullptr) {
   DepArgs a = dep_args(d, buf, src, ns);
+  a.guard = guard;
   const int threads = std::max(64, std::min(256, (h.tuning.dep_threads / 32) * 32));
   // auto (0) = the CTA-per-source pipelined pass: measured fastest at 50k (77 ms per all-source
   // step; the pipelined warp form and the plain CTA form measured 153 and 151 ms, when this pass
@@ -2401,9 +2412,23 @@ static bool dep_reads_hops(const Handle &h) {
   return !(h.host.kind == IndexKind::CSR && (h.tuning.dep_form == 0 || h.tuning.dep_form == 4));
 }
 
-void launch_chunk(const Handle &h, DeviceState *d, const int32_t *d_src_tid, int32_t cnt, int buf, cudaStream_t st) {
-  launch_label(h, d, buf, d_src_tid, cnt, false, st, dep_reads_hops(h));
-  launch_dep(h, d, buf, d_src_tid, cnt, st);
+// The dependency pass runs right after the scan on the same stream: run concurrently on a second
+// stream the two kernels thrash each other's caches and both slow down ~2x.
+void launch_chunk(const Handle &h, DeviceState *d, const int32_t *d_src_tid, int32_t cnt, int buf, cudaStream_t st,
+                  const int32_t *guard) {
+  launch_label(h, d, buf, d_src_tid, cnt, false, st, dep_reads_hops(h), guard);
+  launch_dep(h, d, buf, d_src_tid, cnt, st, false, guard);
+}
+
+void launch_sources(const Handle &h, DeviceState *d, const int32_t *d_src_tid, int32_t ns, cudaStream_t st, bool rerun) {
+  const int32_t *guard = nullptr;
+  if (use_tree(h, d, ns)) {
+    launch_tree(h, d, d_src_tid, ns, st);
+    if (rerun) return;
+    guard = tree_guard(d);
+  }
+  for (int32_t off = 0; off < ns; off += d->chunk)  // stream order frees the buffer for the next chunk
+    launch_chunk(h, d, d_src_tid + off, std::min(d->chunk, ns - off), 0, st, guard);
 }
 
 void launch_tid_to_vid(DeviceState *d, const double *in_tid, double *out_vid, int accumulate, cudaStream_t st) {
@@ -2907,19 +2932,23 @@ struct FillArgs {
   int32_t *dis;
   int2 *ch;
   int32_t *anc;  // H2H only: ancestor id of each entry (the H2H fill reads rows of ancestors below x)
+  int32_t *wrapped;  // set where a path count passes 2^31
 };
 
 // Merge of one separator's candidate into an entry: shorter replaces, equal adds the count and
 // keeps the larger hop (TreeDecomp.cpp:157-193); order-free, so any order of separators gives the
 // sequential merge's entry.
 template <bool MHL>
-__device__ __forceinline__ void fill_merge(int &best, unsigned &c, int &hp, int nd, unsigned nc, int nh) {
+__device__ __forceinline__ void fill_merge(int &best, unsigned &c, int &hp, int nd, unsigned long long nc, int nh,
+                                           unsigned long long &high) {
   if (nd < best) {
     best = nd;
-    c = nc;
+    c = (unsigned)nc;
     hp = nh;
+    if (MHL) high |= nc;
   } else if (MHL && nd == best) {
-    c += nc;
+    high |= nc + c;  // the count before it wraps
+    c += (unsigned)nc;
     hp = max(hp, nh);
   }
 }
@@ -2944,6 +2973,7 @@ struct FillSep {
 template <bool MHL, class GET>
 __device__ __forceinline__ void fill_entry(const FillArgs &f, int j, int64_t ajoff, int nx, GET sep, int &best,
                                            unsigned &c, int &hp) {
+  unsigned long long high = 0;
   for (int i0 = 0; i0 < nx; i0 += kFillBatch) {
     int dv[kFillBatch];
     int2 cv[kFillBatch];
@@ -2963,11 +2993,13 @@ __device__ __forceinline__ void fill_entry(const FillArgs &f, int j, int64_t ajo
     for (int q = 0; q < kFillBatch; q++) {
       if (x[q].k == INT_MIN) continue;
       if (MHL)
-        fill_merge<true>(best, c, hp, x[q].len + dv[q], x[q].cnt * (unsigned)cv[q].x, x[q].hop + cv[q].y);
+        fill_merge<true>(best, c, hp, x[q].len + dv[q], (unsigned long long)x[q].cnt * (unsigned)cv[q].x, x[q].hop + cv[q].y,
+                         high);
       else
-        fill_merge<false>(best, c, hp, x[q].len + dv[q], 0u, 0);
+        fill_merge<false>(best, c, hp, x[q].len + dv[q], 0ull, 0, high);
     }
   }
+  if (MHL && (high >> 31)) *f.wrapped = 1;
 }
 
 // One launch per tree depth k (all its nodes have rows of k entries); a warp takes one node's
@@ -3191,9 +3223,9 @@ static void finish_state(Handle &h, DeviceState *d) {
   alloc_scratch(h, d);
   d->bc_tid = dmalloc<double>(d, ix.n);
   d->bc_vid = dmalloc<double>(d, ix.n);
-  d->err = dmalloc<int32_t>(d, 1);
+  d->err = dmalloc<int32_t>(d, 2);
   d->grid_ctl = dmalloc<int32_t>(d, kGridCtlBytes / 4);
-  CK(cudaMemsetAsync(d->err, 0, 4, st));
+  CK(cudaMemsetAsync(d->err, 0, 8, st));
   CK(cudaStreamSynchronize(st));
 }
 
@@ -3214,15 +3246,38 @@ void device_upload(Handle &h, int device) {
       CK(cudaMemcpyAsync(d->ch, ix.ch.data(), ix.ch.size() * 4, cudaMemcpyHostToDevice, st));
     }
     finish_state(h, d);
+    if (!ix.seps.off.empty()) {  // (an index loaded from a file has none)
+      int64_t *d_soff = nullptr;
+      int4 *d_sep = nullptr;
+      cudaError_t e = cudaMalloc(&d_soff, ix.seps.off.size() * 8);
+      if (e == cudaSuccess) e = cudaMalloc(&d_sep, std::max<size_t>(16, ix.seps.ent.size() * 4));
+      try {
+        if (e == cudaSuccess) {
+          CK(cudaMemcpyAsync(d_soff, ix.seps.off.data(), ix.seps.off.size() * 8, cudaMemcpyHostToDevice, st));
+          if (!ix.seps.ent.empty())
+            CK(cudaMemcpyAsync(d_sep, ix.seps.ent.data(), ix.seps.ent.size() * 4, cudaMemcpyHostToDevice, st));
+          tree_build(h, d, ix.seps.off, d_soff, d_sep);
+        } else {
+          cudaGetLastError();  // no room: the label kernels answer
+        }
+      } catch (...) {
+        cudaFree(d_soff);
+        cudaFree(d_sep);
+        throw;
+      }
+      cudaFree(d_soff);
+      cudaFree(d_sep);
+    }
   } catch (...) {
     device_release(h);
     throw;
   }
 }
 
-void device_build(Handle &h, int device, const Separators &seps) {
+void device_build(Handle &h, int device) {
   NvtxRange nvtx("qbc.build_device");
   Index &ix = h.host;
+  const Separators &seps = ix.seps;
   try {
     DeviceState *d = nullptr;
     {
@@ -3288,12 +3343,12 @@ void device_build(Handle &h, int device, const Separators &seps) {
       }
       CK(cudaMalloc(&d_soff, seps.off.size() * 8));
       CK(cudaMalloc(&d_sep, std::max<size_t>(16, seps.ent.size() * 4)));
-      CK(cudaMalloc(&d_max, 4));
+      CK(cudaMalloc(&d_max, 8));
       CK(cudaMemcpyAsync(d_nodes, nodes.data(), nodes.size() * 4, cudaMemcpyHostToDevice, st));
       CK(cudaMemcpyAsync(d_soff, seps.off.data(), seps.off.size() * 8, cudaMemcpyHostToDevice, st));
       if (!seps.ent.empty()) CK(cudaMemcpyAsync(d_sep, seps.ent.data(), seps.ent.size() * 4, cudaMemcpyHostToDevice, st));
-      CK(cudaMemsetAsync(d_max, 0, 4, st));
-      FillArgs f{d->depth, d->parent, d->lab_off, d_soff, d_sep, d->dis, d->ch, f_anc};
+      CK(cudaMemsetAsync(d_max, 0, 8, st));
+      FillArgs f{d->depth, d->parent, d->lab_off, d_soff, d_sep, d->dis, d->ch, f_anc, d_max + 1};
       if (TraceScope::enabled()) {  // split the phase: buffers and upload, then the fill kernels
         CK(cudaStreamSynchronize(st));
         t_fill = std::make_unique<TraceScope>("device row fill kernels");
@@ -3320,24 +3375,28 @@ void device_build(Handle &h, int device, const Separators &seps) {
       }
       k_max_i32<<<148 * 4, 256, 0, st>>>(d->dis, L, d_max);
       CK(cudaGetLastError());
-      int32_t mx = 0;
-      CK(cudaMemcpyAsync(&mx, d_max, 4, cudaMemcpyDeviceToHost, st));
+      int32_t mx[2] = {0, 0};
+      CK(cudaMemcpyAsync(mx, d_max, 8, cudaMemcpyDeviceToHost, st));
       CK(cudaStreamSynchronize(st));
-      ix.max_label = mx;
+      ix.max_label = mx[0];
+      ix.counts_wrapped = mx[1] != 0;
+      ix.rows_on_host = false;
+      ix.dis.clear();
+      ix.ch.clear();
+      ix.anc.clear();
+      ix.aend.clear();
+      t_fill.reset();
+      {
+        TraceScope t_fin("per-source scratch");
+        finish_state(h, d);
+        if (TraceScope::enabled()) CK(cudaDeviceSynchronize());
+      }
+      tree_build(h, d, seps.off, d_soff, d_sep);
     } catch (...) {
       free_tmp();
       throw;
     }
     free_tmp();
-    ix.rows_on_host = false;
-    ix.dis.clear();
-    ix.ch.clear();
-    ix.anc.clear();
-    ix.aend.clear();
-    t_fill.reset();
-    TraceScope t_fin("per-source scratch");
-    finish_state(h, d);
-    if (TraceScope::enabled()) CK(cudaDeviceSynchronize());
   } catch (...) {
     device_release(h);
     throw;
@@ -3373,6 +3432,7 @@ void device_release(Handle &h) {
                   d->dsrc_tid, d->dsrc_sorted, d->dsrc_tmp};  // dis_sh aliases dis
   for (void *p : ptrs)
     if (p) cudaFree(p);
+  tree_free(d);
   free_scratch(d);
   for (int b = 0; b < 2; b++) {
     if (d->ev_label[b]) cudaEventDestroy(d->ev_label[b]);
@@ -3397,9 +3457,10 @@ DeviceState *need_dev(Handle &h) {
   return h.dev;
 }
 
-void check_err(DeviceState *d) {
-  int32_t e = 0;
-  CK(cudaMemcpy(&e, d->err, 4, cudaMemcpyDeviceToHost));
+bool check_err(DeviceState *d) {
+  int32_t w[2] = {0, 0};
+  CK(cudaMemcpy(w, d->err, 8, cudaMemcpyDeviceToHost));
+  const int32_t e = w[0];
   if (e != ERR_NONE) {
     CK(cudaMemset(d->err, 0, 4));
     throw Error(QBC_EDEVICE, e == ERR_DISCONNECTED ? "device: SP-DAG wave pass did not reach every vertex"
@@ -3408,6 +3469,7 @@ void check_err(DeviceState *d) {
                              : e == ERR_SWEEP_BOUND ? "device: shortest-path sweep ran past its pass bound"
                                                    : "device: kernel error word " + std::to_string(e));
   }
+  return w[1] != 0 && tree_disable(d);
 }
 
 // ------------------------------------------------------------------------------- drivers
@@ -3446,7 +3508,7 @@ static const int32_t *device_sources_tid_order(DeviceState *d, const int32_t *d_
   return d->dsrc_sorted;
 }
 
-void device_bc_sources(Handle &h, const int32_t *d_sources0, int32_t ns, double *d_bc_vid, void *stream) {
+void device_bc_sources(Handle &h, const int32_t *d_sources0, int32_t ns, double *d_bc_vid, void *stream, bool rerun) {
   NvtxRange nvtx("qbc.bc_sources_device");
   DeviceState *d = need_dev(h);
   cudaStream_t user = stream ? (cudaStream_t)stream : d->s_label;
@@ -3457,14 +3519,7 @@ void device_bc_sources(Handle &h, const int32_t *d_sources0, int32_t ns, double 
   CK(cudaEventRecord(d->ev_label[1], d->s_label));
   CK(cudaStreamWaitEvent(d->s_dep, d->ev_label[1], 0));
   const int32_t *tids = ns > 0 ? device_sources_tid_order(d, d_sources0, ns, d->s_label) : nullptr;
-  for (int32_t off = 0; off < ns; off += d->chunk) {
-    const int b = 0;  // stream order frees the buffer for the next chunk
-    const int32_t cnt = std::min(d->chunk, ns - off);
-    launch_label(h, d, b, tids + off, cnt, false, d->s_label, dep_reads_hops(h));
-    // The dependency pass runs right after the scan on the same stream: run concurrently on a
-    // second stream the two kernels thrash each other's caches and both slow down ~2x.
-    launch_dep(h, d, b, tids + off, cnt, d->s_label);
-  }
+  if (ns > 0) launch_sources(h, d, tids, ns, d->s_label, rerun);
   CK(cudaEventRecord(d->ev_dep[0], d->s_label));
   CK(cudaStreamWaitEvent(user, d->ev_dep[0], 0));
   k_tid_to_vid_f64<<<(d->n + 255) / 256, 256, 0, user>>>(d->bc_tid, d->vid_of, d_bc_vid, d->n, 1);
@@ -3544,11 +3599,12 @@ void host_bc_sources(Handle &h, const int32_t *sources0, int32_t ns, double *bc_
   DeviceState *d = need_dev(h);
   std::vector<int32_t> srt = tid_sorted(h.host, sources0, ns);
   int32_t *ds = stage_sources(d, srt.data(), ns, d->n);
-  CK(cudaMemsetAsync(d->bc_vid, 0, (size_t)d->n * 8, d->s_label));
-  device_bc_sources(h, ds, ns, d->bc_vid, d->s_label);
-  CK(cudaMemcpyAsync(bc_out, d->bc_vid, (size_t)d->n * 8, cudaMemcpyDeviceToHost, d->s_label));
-  CK(cudaStreamSynchronize(d->s_label));
-  check_err(d);
+  do {
+    CK(cudaMemsetAsync(d->bc_vid, 0, (size_t)d->n * 8, d->s_label));
+    device_bc_sources(h, ds, ns, d->bc_vid, d->s_label, true);
+    CK(cudaMemcpyAsync(bc_out, d->bc_vid, (size_t)d->n * 8, cudaMemcpyDeviceToHost, d->s_label));
+    CK(cudaStreamSynchronize(d->s_label));
+  } while (check_err(d));
 }
 
 void host_bc_plain(Handle &h, const int32_t *sources0, int32_t ns, double *bc_out) {

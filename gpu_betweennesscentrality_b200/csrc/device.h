@@ -43,8 +43,9 @@ void device_upload(Handle &h, int device);
 // The last dt.r vertices of a min-degree elimination on the device (a dense matrix, one pick and
 // one shortcut update per step); fills dt.order / dt.x_off / dt.x.
 void device_dense_eliminate(int device, DenseTail &dt);
-// Uploads the index structure and fills its label rows on the device (host rows stay empty).
-void device_build(Handle &h, int device, const Separators &seps);
+// Uploads the index structure and fills its label rows on the device from the index's separators
+// (host rows stay empty).
+void device_build(Handle &h, int device);
 // Copies device-built label rows to the host index (no-op when they are there already).
 void device_download_rows(Handle &h);
 void device_release(Handle &h);
@@ -55,7 +56,9 @@ int device_id(const Handle &h);  // -1 when not uploaded
 
 // BC over `sources0` (0-based vids) accumulated into d_bc_vid (n doubles, vid order, device).
 // Enqueued on `stream` (nullptr: the handle's stream); the caller synchronises.
-void device_bc_sources(Handle &h, const int32_t *d_sources0, int32_t ns, double *d_bc_vid, void *stream);
+// rerun: as for launch_sources (device_state.h).
+void device_bc_sources(Handle &h, const int32_t *d_sources0, int32_t ns, double *d_bc_vid, void *stream,
+                       bool rerun = false);
 // Same with host source list and host output (overwritten); synchronous.
 void host_bc_sources(Handle &h, const int32_t *sources0, int32_t ns, double *bc_out);
 // plain path: one source per launch pair

@@ -58,6 +58,7 @@ struct RowView {
 
 // ------------------------------------------------------------------------------- state
 struct SweepCache;  // captured sweep graphs (sweep.cu)
+struct TreePlan;    // BC over the elimination tree (tree.cu)
 
 struct DeviceState {
   int device = 0;
@@ -96,7 +97,7 @@ struct DeviceState {
   void *dsrc_tmp = nullptr;
   size_t dsrc_tmp_bytes = 0;
   int32_t dsrc_cap = 0;
-  int32_t *err = nullptr;
+  int32_t *err = nullptr;       // error word, then the tree sweeps' wrap word
   int32_t *grid_ctl = nullptr;  // control block of the cooperative plain sweep (kGridCtlBytes)
   int64_t bytes = 0, scratch_bytes = 0;
   int smem_optin = 0;
@@ -107,6 +108,7 @@ struct DeviceState {
   double label_ms = 0.0, dep_ms = 0.0;
   int64_t label_launches = 0, dep_launches = 0, launches = 0;
   SweepCache *sweep = nullptr;
+  TreePlan *tree = nullptr;  // null: the index has no separators, or its keys or counts do not fit
 };
 
 static std::pair<cudaEvent_t, cudaEvent_t> take_events(std::vector<std::pair<cudaEvent_t, cudaEvent_t>> &pool,
@@ -139,7 +141,22 @@ static T *dupload(DeviceState *d, const std::vector<T> &v, cudaStream_t s) {
 // Launches of one chunk of sources (their tids at d_src_tid, cnt <= chunk) on stream st, using
 // scratch buffer `buf`: the label scan, then the dependency pass, which adds 0.5 * delta into
 // d->bc_tid (not cleared here).  Nothing in it synchronises, so it can be stream-captured.
-void launch_chunk(const Handle &h, DeviceState *d, const int32_t *d_src_tid, int32_t cnt, int buf, cudaStream_t st);
+// guard (may be null): the kernels leave at once while *guard is 0.
+void launch_chunk(const Handle &h, DeviceState *d, const int32_t *d_src_tid, int32_t cnt, int buf, cudaStream_t st,
+                  const int32_t *guard = nullptr);
+// The chunks of a whole source list (ns tids at d_src_tid), its BC added into d->bc_tid: over the
+// elimination tree where use_tree holds, else chunk by chunk with the label or sweep kernels.
+// rerun: the caller synchronises afterwards and repeats the call when check_err says so; without
+// it the label kernels follow the tree's, guarded by its wrap word.
+void launch_sources(const Handle &h, DeviceState *d, const int32_t *d_src_tid, int32_t ns, cudaStream_t st, bool rerun);
+// BC over the elimination tree (tree.cu)
+void tree_build(Handle &h, DeviceState *d, const std::vector<int64_t> &soff, const int64_t *d_soff, const int4 *d_sep);
+void tree_free(DeviceState *d);
+bool use_tree(const Handle &h, const DeviceState *d, int32_t ns);
+const int32_t *tree_guard(const DeviceState *d);
+// no call uses the plan after this; false when none did
+bool tree_disable(DeviceState *d);
+void launch_tree(const Handle &h, DeviceState *d, const int32_t *d_src_tid, int32_t ns, cudaStream_t st);
 // CSR index: rows of ns sources by shortest-path sweeps into the given scratch (rec/hop/order/lcnt
 // laid out as a buffer of ns slots), one CTA per source (sssp.cu): records (dist, count, 0), hop
 // layers and, when maxhop is not null, the largest layer per source -- the label scan's outputs.
@@ -160,7 +177,8 @@ void launch_vid_to_tid(DeviceState *d, const int32_t *vids, int32_t *tids, int32
 DeviceState *need_dev(Handle &h);
 // frees the captured sweep graphs (they hold scratch pointers; called whenever scratch changes)
 void sweep_cache_free(DeviceState *d);
-// reads and clears the device error word; throws QBC_EDEVICE when a kernel set it (synchronous)
-void check_err(DeviceState *d);
+// reads and clears the device error word; throws QBC_EDEVICE when a kernel set it (synchronous).
+// True when a path count wrapped in a tree sweep since the last call: its results are void.
+bool check_err(DeviceState *d);
 
 }  // namespace qbc

@@ -578,6 +578,28 @@ void fill_ancestor_rows(Index &ix) {
   }
 }
 
+// separator lists of an elimination in tid space
+static Separators separators_of(const Elimination &el, const Index &ix) {
+  Separators seps;
+  const int32_t n = ix.n;
+  std::vector<int64_t> xs((size_t)n, 0);
+  for (int32_t s = 0; s < n; s++) xs[ix.tid_of[el.order[s]]] = s;
+  seps.off.assign((size_t)n + 1, 0);
+  for (int32_t t = 0; t < n; t++) seps.off[t + 1] = seps.off[t] + (el.x_off[xs[t] + 1] - el.x_off[xs[t]]);
+  seps.ent.assign((size_t)seps.off[n] * 4, 0);
+  for (int32_t t = 0; t < n; t++) {
+    int64_t o = seps.off[t] * 4;
+    for (int64_t i = el.x_off[xs[t]]; i < el.x_off[xs[t] + 1]; i++) {
+      const Adj &a = el.x[i];
+      seps.ent[o++] = ix.tid_of[a.v];
+      seps.ent[o++] = a.len;
+      seps.ent[o++] = (int32_t)a.cnt;
+      seps.ent[o++] = a.hop;
+    }
+  }
+  return seps;
+}
+
 // Elimination (min-degree for MHL, the order file's for H2H) and tree, without label rows; the
 // separator list of each tree node goes to `seps` in tid space for the device row fill.
 Index prepare_index(const Graph &g, IndexKind kind, const std::vector<int32_t> *node_order, Separators &seps,
@@ -600,22 +622,7 @@ Index prepare_index(const Graph &g, IndexKind kind, const std::vector<int32_t> *
   ix.kind = kind;
   TraceScope t("tree and separators");
   make_tree(g, el, ix, false);
-  const int32_t n = g.n;
-  std::vector<int64_t> xs((size_t)n, 0);
-  for (int32_t s = 0; s < n; s++) xs[ix.tid_of[el.order[s]]] = s;
-  seps.off.assign((size_t)n + 1, 0);
-  for (int32_t t = 0; t < n; t++) seps.off[t + 1] = seps.off[t] + (el.x_off[xs[t] + 1] - el.x_off[xs[t]]);
-  seps.ent.assign((size_t)seps.off[n] * 4, 0);
-  for (int32_t t = 0; t < n; t++) {
-    int64_t o = seps.off[t] * 4;
-    for (int64_t i = el.x_off[xs[t]]; i < el.x_off[xs[t] + 1]; i++) {
-      const Adj &a = el.x[i];
-      seps.ent[o++] = ix.tid_of[a.v];
-      seps.ent[o++] = a.len;
-      seps.ent[o++] = (int32_t)a.cnt;
-      seps.ent[o++] = a.hop;
-    }
-  }
+  seps = separators_of(el, ix);
   return ix;
 }
 
@@ -624,14 +631,17 @@ Index build_mhl(const Graph &g, int nthreads) {
   Index ix;
   ix.kind = IndexKind::MHL;
   make_tree(g, el, ix);
+  ix.seps = separators_of(el, ix);
   const int64_t L = ix.lab_off[g.n];
   ix.dis.assign((size_t)L, 0);
   ix.ch.assign((size_t)L * 2, 0);
   // separator list of each tid: (tid of x_i, len, cnt, hop)
   std::vector<int64_t> xs((size_t)g.n + 1, 0);
   for (int32_t s = 0; s < g.n; s++) xs[ix.tid_of[el.order[s]]] = s;
+  std::atomic<bool> wrapped{false};
   fill_rows(ix, hardware_threads(nthreads), [&](int32_t p, auto &&wait) {
     const int32_t h = ix.depth[p];
+    uint64_t high = 0;  // counts before they wrap
     int32_t *dis = ix.dis.data() + ix.lab_off[p];
     int32_t *ch = ix.ch.data() + 2 * ix.lab_off[p];
     for (int32_t j = 0; j < h - 1; j++) { dis[j] = kInf; ch[2 * j] = 0; ch[2 * j + 1] = 0; }
@@ -648,16 +658,20 @@ Index build_mhl(const Graph &g, int nthreads) {
       const int32_t *xc = ix.ch.data() + 2 * ix.lab_off[xt];
       for (int32_t j = 0; j <= k; j++) {
         const int32_t nd = a.len + xd[j];
-        const uint32_t nc = a.cnt * (uint32_t)xc[2 * j];
+        const uint64_t wide = (uint64_t)a.cnt * (uint32_t)xc[2 * j];
+        const uint32_t nc = (uint32_t)wide;
         const int32_t nh = a.hop + xc[2 * j + 1];
-        if (nd < dis[j]) { dis[j] = nd; ch[2 * j] = (int32_t)nc; ch[2 * j + 1] = nh; }
+        if (nd < dis[j]) { dis[j] = nd; ch[2 * j] = (int32_t)nc; ch[2 * j + 1] = nh; high |= wide; }
         else if (nd == dis[j]) {
+          high |= wide + (uint32_t)ch[2 * j];
           ch[2 * j] = (int32_t)((uint32_t)ch[2 * j] + nc);
           if (nh > ch[2 * j + 1]) ch[2 * j + 1] = nh;
         }
       }
     }
+    if (high >> 31) wrapped.store(true, std::memory_order_relaxed);
   });
+  ix.counts_wrapped = wrapped.load();
   ix.max_label = 0;
   for (int32_t t = 0; t < ix.n; t++)
     for (int32_t j = 0; j < ix.depth[t]; j++) ix.max_label = std::max(ix.max_label, ix.dis[ix.lab_off[t] + j]);
@@ -678,6 +692,7 @@ Index build_h2h(const Graph &g, const std::vector<int32_t> &node_order, int nthr
   Index ix;
   ix.kind = IndexKind::H2H;
   make_tree(g, el, ix);
+  ix.seps = separators_of(el, ix);
   const int64_t L = ix.lab_off[g.n];
   ix.dis.assign((size_t)L, 0);
   std::vector<int64_t> xs((size_t)g.n + 1, 0);

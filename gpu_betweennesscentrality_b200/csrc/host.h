@@ -70,6 +70,13 @@ std::vector<int32_t> read_query(const std::string &path, int32_t n);
 // shortest-path sweeps over the arc list.
 enum class IndexKind : int { MHL = 0, H2H = 1, CSR = 2 };
 
+// Separator lists in tid space, for the device row fill and the tree plan: node t's entries are
+// ent[4*off[t] .. 4*off[t+1]), each (tid of x, shortcut length, path count bits, max hop), in
+// elimination order of the separator.
+struct Separators {
+  std::vector<int64_t> off;
+  std::vector<int32_t> ent;
+};
 // Tree-decomposition index in DFS-preorder numbering ("tid").  Row p holds one entry per
 // ancestor, root first, plus the node itself last (dis 0, cnt 1, hop 0); rows start on 4-entry
 // boundaries so 16-byte vector loads stay aligned.
@@ -91,16 +98,11 @@ struct Index {
   // arcs in tid space, each tail's arcs in file order
   std::vector<int32_t> arc_off, arc_head, arc_w;
   int64_t depth_sum = 0;
+  Separators seps;           // empty for an index loaded from a file (and for CSR)
+  bool counts_wrapped = false;  // a label's path count passed 2^31 when the rows were filled
   bool rows_on_host = true;  // false: label rows (dis/ch/anc/aend) exist only on the device
 };
 
-// Separator lists in tid space, for the device row fill: node t's entries are
-// ent[4*off[t] .. 4*off[t+1]), each (tid of x, shortcut length, path count bits, max hop), in
-// elimination order of the separator.
-struct Separators {
-  std::vector<int64_t> off;
-  std::vector<int32_t> ent;
-};
 // The last r vertices of a min-degree elimination, handed to another engine (the device's dense
 // elimination, device_dense_eliminate): the vertices still present, ascending (local id = index),
 // with their current adjacency in local ids.  The engine returns the rest of the elimination: the

@@ -60,7 +60,7 @@ uint64_t fnv(uint64_t h, const void *p, size_t bytes) {
 
 uint64_t tuning_key(const Handle &h, const DeviceState *d) {
   const Tuning &t = h.tuning;
-  const int32_t f[] = {t.lanes_per_source, t.label_threads, t.split, t.dep_threads, t.dep_form, t.queue_depth, t.label_warps, t.label_tile, t.label_passes, t.sweep_delta, t.sweep_threads, t.label_sources, t.label_stream, d->chunk};
+  const int32_t f[] = {t.lanes_per_source, t.label_threads, t.split, t.dep_threads, t.dep_form, t.queue_depth, t.label_warps, t.label_tile, t.label_passes, t.sweep_delta, t.sweep_threads, t.label_sources, t.label_stream, d->chunk, d->tree ? 1 : 0};
   return fnv(1469598103934665603ull, f, sizeof(f));
 }
 
@@ -161,6 +161,14 @@ void sweep_cache_free(DeviceState *d) {
   d->sweep = nullptr;
 }
 
+// Whether a path count of the sweep just finished wrapped: its captured graphs then go, and the
+// call is repeated with the label kernels.
+static bool sweep_wrapped(DeviceState *d) {
+  if (!check_err(d)) return false;
+  sweep_cache_free(d);
+  return true;
+}
+
 static constexpr size_t kMaxPlans = 4;
 
 static SweepPlan &plan_for(Handle &h, DeviceState *d, const int32_t *sources0, int32_t ns) {
@@ -194,7 +202,7 @@ static SweepPlan &plan_for(Handle &h, DeviceState *d, const int32_t *sources0, i
     int32_t *dt = p->d_tids;
     p->whole = capture(d, st, p->per_replay, [&] {
       CK(cudaMemsetAsync(d->bc_tid, 0, (size_t)d->n * 8, st));
-      for (int32_t off = 0; off < total; off += d->chunk) launch_chunk(h, d, dt + off, std::min(d->chunk, total - off), 0, st);
+      if (total > 0) launch_sources(h, d, dt, total, st, true);
     });
   } catch (...) {
     free_plan(p.get());
@@ -207,13 +215,14 @@ static SweepPlan &plan_for(Handle &h, DeviceState *d, const int32_t *sources0, i
 void host_bc_sweep(Handle &h, const int32_t *sources0, int32_t ns, double *bc_out) {
   NvtxRange nvtx("qbc.bc_sweep");
   DeviceState *d = need_dev(h);
-  SweepPlan &p = plan_for(h, d, sources0, ns);
   cudaStream_t st = d->s_label;
-  replay(d, p.whole, p.per_replay, st);
-  launch_tid_to_vid(d, d->bc_tid, d->bc_vid, 0, st);
-  CK(cudaMemcpyAsync(bc_out, d->bc_vid, (size_t)d->n * 8, cudaMemcpyDeviceToHost, st));
-  CK(cudaStreamSynchronize(st));
-  check_err(d);
+  do {
+    SweepPlan &p = plan_for(h, d, sources0, ns);
+    replay(d, p.whole, p.per_replay, st);
+    launch_tid_to_vid(d, d->bc_tid, d->bc_vid, 0, st);
+    CK(cudaMemcpyAsync(bc_out, d->bc_vid, (size_t)d->n * 8, cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+  } while (sweep_wrapped(d));
 }
 
 void host_query_batch(Handle &h, const int32_t *points0, int64_t total, const int32_t *sources0, int32_t ns, double *out) {
@@ -221,31 +230,32 @@ void host_query_batch(Handle &h, const int32_t *points0, int64_t total, const in
   DeviceState *d = need_dev(h);
   for (int64_t i = 0; i < total; i++)
     if (points0[i] < 0 || points0[i] >= h.host.n) throw Error(QBC_EINVAL, "query id " + std::to_string(points0[i]) + " out of range");
-  SweepPlan &p = plan_for(h, d, sources0, ns);
-  SweepCache &c = *d->sweep;
-  cudaStream_t st = d->s_label;
-  if (total > c.points_cap) {
+  do {
+    SweepPlan &p = plan_for(h, d, sources0, ns);
+    SweepCache &c = *d->sweep;
+    cudaStream_t st = d->s_label;
+    if (total > c.points_cap) {
+      CK(cudaStreamSynchronize(st));
+      if (c.d_points) cudaFree(c.d_points);
+      if (c.d_out) cudaFree(c.d_out);
+      c.d_points = nullptr;
+      c.d_out = nullptr;
+      c.points_cap = 0;
+      CK(cudaMalloc(&c.d_points, (size_t)total * 4));
+      CK(cudaMalloc(&c.d_out, (size_t)total * 8));
+      c.points_cap = total;
+    }
+    if (total) CK(cudaMemcpyAsync(c.d_points, points0, (size_t)total * 4, cudaMemcpyHostToDevice, st));
+    replay(d, p.whole, p.per_replay, st);
+    if (total) {
+      const int blocks = (int)std::min<int64_t>(148 * 4, (total + 255) / 256);
+      k_pick<<<blocks, 256, 0, st>>>(d->bc_tid, d->tid_of, c.d_points, (int32_t)total, d->n, c.d_out, d->err);
+      CK(cudaGetLastError());
+      d->launches++;
+      CK(cudaMemcpyAsync(out, c.d_out, (size_t)total * 8, cudaMemcpyDeviceToHost, st));
+    }
     CK(cudaStreamSynchronize(st));
-    if (c.d_points) cudaFree(c.d_points);
-    if (c.d_out) cudaFree(c.d_out);
-    c.d_points = nullptr;
-    c.d_out = nullptr;
-    c.points_cap = 0;
-    CK(cudaMalloc(&c.d_points, (size_t)total * 4));
-    CK(cudaMalloc(&c.d_out, (size_t)total * 8));
-    c.points_cap = total;
-  }
-  if (total) CK(cudaMemcpyAsync(c.d_points, points0, (size_t)total * 4, cudaMemcpyHostToDevice, st));
-  replay(d, p.whole, p.per_replay, st);
-  if (total) {
-    const int blocks = (int)std::min<int64_t>(148 * 4, (total + 255) / 256);
-    k_pick<<<blocks, 256, 0, st>>>(d->bc_tid, d->tid_of, c.d_points, (int32_t)total, d->n, c.d_out, d->err);
-    CK(cudaGetLastError());
-    d->launches++;
-    CK(cudaMemcpyAsync(out, c.d_out, (size_t)total * 8, cudaMemcpyDeviceToHost, st));
-  }
-  CK(cudaStreamSynchronize(st));
-  check_err(d);
+  } while (sweep_wrapped(d));
 }
 
 // ------------------------------------------------------------------------------- autotune
@@ -260,7 +270,7 @@ static double time_sample(Handle &h, DeviceState *d, const int32_t *d_tids, int3
     for (int r = -1; r < reps; r++) {
       CK(cudaMemsetAsync(d->bc_tid, 0, (size_t)d->n * 8, st));
       CK(cudaEventRecord(a, st));
-      for (int32_t off = 0; off < ns; off += d->chunk) launch_chunk(h, d, d_tids + off, std::min(d->chunk, ns - off), 0, st);
+      launch_sources(h, d, d_tids, ns, st, false);
       CK(cudaEventRecord(b, st));
       CK(cudaEventSynchronize(b));
       float ms = 0.f;
@@ -705,7 +715,7 @@ Server *serve_open(Handle &h, const int32_t *sources0, int32_t ns, const int64_t
       Server *sp = s.get();
       s->graphs.push_back(capture(d, s->st, s->per_chunk, [&] {
         CK(cudaMemsetAsync(d->bc_tid, 0, (size_t)d->n * 8, sp->st));
-        launch_chunk(h, d, sp->d_tids + off, cnt, 0, sp->st);
+        launch_sources(h, d, sp->d_tids + off, cnt, sp->st, false);
         k_gather_entries<<<148 * 2, 256, 0, sp->st>>>(d->bc_tid, sp->d_ent, sp->d_count, sp->d_acc);
         CK(cudaGetLastError());
         d->launches++;
