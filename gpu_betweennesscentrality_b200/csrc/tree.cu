@@ -39,6 +39,7 @@
 #include <algorithm>
 #include <climits>
 #include <cstdlib>
+#include <type_traits>
 
 #include "device_state.h"
 
@@ -50,14 +51,14 @@ constexpr unsigned kAll = 0xffffffffu;
 constexpr unsigned kNoKey = 0xffffffffu;
 constexpr int kGroup = 64;           // sources a warp takes: two neighbouring ones per lane
 constexpr int kPieceLen = 32;        // trunk vertices per piece
-constexpr int kBottomRows = 32;      // shared-memory rows of a bottom subtree (its separator + its vertices)
-constexpr int kBottomEdges = 160;    // ... and its edges (grids of 2k to 1M vertices: at most 100)
-constexpr int kInPieceEdges = kPieceLen * (kPieceLen - 1) / 2;
+constexpr int kBottomRows = 24;      // shared-memory rows of a bottom subtree (its separator + its vertices)
+constexpr int kBottomEdges = 128;    // ... and its edges (grids of 2k to 1M vertices: at most 74)
 constexpr int kMaxUnpackLevels = 1024;
 
 struct TreeArgs {
   int n, H, NT, bits;
   unsigned dist_lim;               // distances of shortest paths are below it
+  unsigned absent;                 // key of a missing entry: above every distance
   const int32_t *xoff;             // [n + 1] edge range of a vertex
   const int2 *ex;                  // per edge (x: trunk index or bottom row, (L << bits) | (i + 1))
   const int4 *eup;                 // per edge (depth(x) - 1, L, path count, tid of x)
@@ -123,10 +124,6 @@ __device__ __forceinline__ void lane_sources(const TreeArgs &a, int g, int lane,
 // The minimum of a pair is kept as two keys, (distance, entry index) and the same with the index
 // complemented; their indices differ where several entries reach it.  arg = smallest index |
 // largest << 16: equal for one entry, smallest < largest for exactly two, swapped for more.
-__device__ __forceinline__ void key_min(unsigned &m1, unsigned &m2, unsigned v, unsigned mask) {
-  m1 = min(m1, v);
-  m2 = min(m2, v ^ mask);
-}
 __device__ __forceinline__ void key_min2(unsigned &m1, unsigned &m2, unsigned v, unsigned w, unsigned mask) {
   m1 = __vimin3_u32(m1, v, w);
   m2 = __vimin3_u32(m2, v ^ mask, w ^ mask);
@@ -445,37 +442,47 @@ __device__ __forceinline__ void add_flows(const TreeArgs &a, int e0, int (&idx)[
   }
 }
 
-// ------------------------------------------------------------------------------- trunk down
-// A CTA takes one piece (a path of at most 32 trunk vertices) for one group.  The minima over the
-// separator vertices above the piece are independent, a warp per vertex (or part of its list); then
-// one warp follows the path in shared memory.  Bound by the latency of those steps (5 M warp
-// instructions in 18 us per 10k list entries and 64 groups at 50k): two groups per CTA, whose 114
-// registers left 16 warps per SM, took 1,602 against 1,005 us for the seven wide levels.
-struct PieceShared {
-  int2 ine[kInPieceEdges];  // edges inside the piece: (kGroup * position, key)
-  int ineC[kInPieceEdges];
-  int inoff[kPieceLen + 1];
-  int4 meta[kPieceLen];
-  int2 sub[kPieceLen];
+// ------------------------------------------------------------------------------- trunk, wide levels
+// A CTA takes one piece (a path of at most PL trunk vertices) for one group of sources.  The minima
+// over the separator vertices above the piece are independent, a warp per vertex; then one warp
+// follows the path over the edges inside the piece in shared memory, while other CTAs fill the SM:
+// levels with many pieces are bound by instructions and occupancy, not by the latency of the path.
+// Pieces of up to 8 and 16 vertices, most of those below the top, have launches of their own with
+// less shared memory and fewer warps to wait for the one on the path.
+template <int PL>
+struct Wide {
+  static constexpr int warps = PL == 8 ? 2 : 4;
 };
 
-__device__ __forceinline__ void load_piece(const TreeArgs &a, int start, int len, PieceShared &p) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+template <int PL>
+struct PieceShared {
+  int2 ine[PL * (PL - 1) / 2];  // edges inside the piece: (kGroup * position, key)
+  int ineC[PL * (PL - 1) / 2];
+  int inoff[PL + 1];
+  int4 meta[PL];
+  int2 sub[PL];
+};
+
+template <int PL>
+__device__ __forceinline__ void load_piece(const TreeArgs &a, int start, int len, PieceShared<PL> &p) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (warp == 0) {
     const int4 m = lane < len ? a.tmeta[start + lane] : make_int4(0, 0, 0, 0);
-    p.meta[lane] = m;
-    if (lane < len) p.sub[lane] = a.tsub[start + lane];
+    if (lane < len) {
+      p.meta[lane] = m;
+      p.sub[lane] = a.tsub[start + lane];
+    }
     int x = m.z;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int z = __shfl_up_sync(kAll, x, o);
       if (lane >= o) x += z;
     }
-    p.inoff[lane] = x - m.z;
-    if (lane == 31) p.inoff[32] = x;
+    if (lane <= len && lane < PL) p.inoff[lane] = x - m.z;
+    if (lane == len - 1) p.inoff[len] = x;
   }
   __syncthreads();
-  for (int i = warp; i < len; i += nw) {
+  for (int i = warp; i < len; i += Wide<PL>::warps) {
     const int4 m = p.meta[i];
     if (lane < m.z) {  // at most 31 edges
       const int2 v = a.ex[m.y - m.z + lane];
@@ -485,247 +492,295 @@ __device__ __forceinline__ void load_piece(const TreeArgs &a, int start, int len
   }
 }
 
-template <int GB>
-__global__ void __launch_bounds__(512) k_trunk_down(TreeArgs a, int piece0, int pl) {
-  extern __shared__ uint32_t sm_td[];
-  __shared__ PieceShared p;
-  constexpr int K = 2 * GB, E = 8 / GB;  // values per lane, edges loaded together
-  if (__syncthreads_or(wrapped(a))) return;
-  const int4 pc = a.piece[piece0 + blockIdx.x];
-  const int start = pc.x, len = pc.y - pc.x;
-  const int g0 = blockIdx.y * GB;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  const unsigned mask = (1u << a.bits) - 1u;
-  const int parts = max(1, min(8, nw / len));  // few vertices: several warps share a list
-  const int gs = pl * kGroup;                  // a group's values in shared memory
-  uint32_t *k1 = sm_td + 2 * lane, *k2 = k1 + GB * gs, *sg = k2 + GB * gs;
-  if (parts > 1)
-    for (int q = threadIdx.x; q < 2 * GB * gs; q += blockDim.x) sm_td[q] = kNoKey;
-  int s[K];
-  size_t gt[GB], gu[GB];  // this lane's place in a group's trunk and U rows (a missing group repeats the last)
+// Minimum keys of a vertex over its entries [e, ee) above the piece, eight or four loaded together.
+__device__ __forceinline__ void scan_above(const TreeArgs &a, int e, int ee, size_t gt, unsigned mask, unsigned (&m1)[2],
+                                           unsigned (&m2)[2]) {
+  if (e >= ee) return;
+  const uint32_t *D = a.D + gt;
+  int2 w[8];  // the next entries, in flight while the current distances are loaded
 #pragma unroll
-  for (int w = 0; w < GB; w++) {
-    const int g = min(g0 + w, a.ng - 1);
-    bool live[2];
-    int sw[2];
-    lane_sources(a, g, lane, sw, live);
-    s[2 * w] = sw[0];
-    s[2 * w + 1] = sw[1];
-    gt[w] = (size_t)g * a.NT * kGroup + 2 * lane;
-    gu[w] = (size_t)g * a.H * kGroup + 2 * lane;
-  }
-  load_piece(a, start, len, p);
-  __syncthreads();
-  for (int task = warp; task < len * parts; task += nw) {
-    const int i = task / parts, part = task - i * parts;
-    const int4 m = p.meta[i];
-    unsigned m1[K], m2[K];
+  for (int q = 0; q < 8; q++) w[q] = __ldg(a.ex + min(e + q, ee - 1));
+  auto step = [&](auto count) {  // (the last entry may repeat)
+    constexpr int N = decltype(count)::value;
+    uint2 d[N];
+    unsigned key[N];
 #pragma unroll
-    for (int k = 0; k < K; k++) {
-      const int2 sub = p.sub[i];
-      m1[k] = up_key(a, part == 0 && m.w <= s[k] && s[k] < sub.x, gu[k >> 1] + (size_t)sub.y * kGroup + (k & 1));
-      m2[k] = m1[k] == kNoKey ? kNoKey : m1[k] ^ mask;
+    for (int q = 0; q < N; q++) {
+      d[q] = *reinterpret_cast<const uint2 *>(D + (size_t)w[q].x * kGroup);
+      key[q] = (unsigned)w[q].y;
     }
-    const int nx = m.y - m.z - m.x, per = ((nx + parts - 1) / parts + 7) & ~7;
-    const int ee = m.x + min(nx, (part + 1) * per);
-    for (int e = m.x + min(nx, part * per); e < ee; e += E) {  // (the last entry may repeat)
-      int2 v[E];
-      uint2 d[E][GB];
+    e += N;
+    if (e < ee) {
 #pragma unroll
-      for (int q = 0; q < E; q++) v[q] = __ldg(a.ex + min(e + q, ee - 1));
-#pragma unroll
-      for (int q = 0; q < E; q++)
-#pragma unroll
-        for (int w = 0; w < GB; w++) d[q][w] = *reinterpret_cast<const uint2 *>(a.D + gt[w] + (size_t)v[q].x * kGroup);
-#pragma unroll
-      for (int q = 0; q < E; q += 2)
-#pragma unroll
-        for (int w = 0; w < GB; w++) {
-          key_min2(m1[2 * w], m2[2 * w], d[q][w].x + (unsigned)v[q].y, d[q + 1][w].x + (unsigned)v[q + 1].y, mask);
-          key_min2(m1[2 * w + 1], m2[2 * w + 1], d[q][w].y + (unsigned)v[q].y, d[q + 1][w].y + (unsigned)v[q + 1].y, mask);
-        }
+      for (int q = 0; q < N; q++) w[q] = __ldg(a.ex + min(e + q, ee - 1));
     }
 #pragma unroll
-    for (int w = 0; w < GB; w++) {
-      const int o = w * gs + i * kGroup;
-      if (parts > 1) {
+    for (int q = 0; q < N; q += 2) {
+      key_min2(m1[0], m2[0], d[q].x + key[q], d[q + 1].x + key[q + 1], mask);
+      key_min2(m1[1], m2[1], d[q].y + key[q], d[q + 1].y + key[q + 1], mask);
+    }
+  };
+  while (e + 4 < ee) step(std::integral_constant<int, 8>{});
+  if (e < ee) step(std::integral_constant<int, 4>{});
+}
+
+// Counts of a minimum over the entries above the piece (first edge e0, nx of them), its argument
+// being smallest | largest << 16; hits: how many entries reach it.
+__device__ __forceinline__ void count_above(const TreeArgs &a, int e0, int nx, size_t gt, size_t gu, unsigned mask,
+                                            const unsigned (&md)[2], const unsigned (&ar)[2], uint32_t (&cnt)[2],
+                                            unsigned (&hits)[2], unsigned &over) {
+  int lo = INT_MAX, hi = 0;
+  bool tie = false;
 #pragma unroll
-        for (int k = 0; k < 2; k++) {
-          atomicMin(k1 + o + k, m1[2 * w + k]);
-          atomicMin(k2 + o + k, m2[2 * w + k]);
-        }
-      } else {
-        *reinterpret_cast<uint2 *>(k1 + o) = make_uint2(m1[2 * w], m1[2 * w + 1]);
-        *reinterpret_cast<uint2 *>(k2 + o) = make_uint2(m2[2 * w], m2[2 * w + 1]);
-      }
+  for (int k = 0; k < 2; k++) {
+    const int a1 = (int)(ar[k] & 0xffff), a2 = (int)(ar[k] >> 16);
+    hits[k] = a1 <= nx;  // (none: no entry above the piece)
+    const int e = e0 + a1 - 1;
+    unsigned long long c = 0;
+    if (a1 == 0) c = a.Uc[gu + k];
+    else if (a1 <= nx) c = (unsigned long long)(unsigned)a.eC[e] * a.S[gt + (size_t)a.ex[e].x * kGroup + k];
+    over |= c > 0x7fffffffull;
+    cnt[k] = (uint32_t)c;
+    if (a1 != a2 && a1 <= nx) {
+      tie = true;
+      lo = min(lo, a1 + 1);
+      hi = max(hi, min(a2, nx));
     }
   }
-  __syncthreads();
-  // along the piece, a warp per group: k1 becomes the distance, k2 the argument
-  if (warp < GB) {
-    uint32_t *r1 = k1 + warp * gs, *r2 = k2 + warp * gs;
-    for (int i = 0; i < len; i++) {
-      uint2 m1 = *reinterpret_cast<uint2 *>(r1 + i * kGroup), m2 = *reinterpret_cast<uint2 *>(r2 + i * kGroup);
-#pragma unroll 4
-      for (int k = p.inoff[i]; k < p.inoff[i + 1]; k++) {
-        const int2 v = p.ine[k];
-        const uint2 d = *reinterpret_cast<uint2 *>(r1 + v.x);
-        key_min(m1.x, m2.x, d.x + (unsigned)v.y, mask);
-        key_min(m1.y, m2.y, d.y + (unsigned)v.y, mask);
-      }
-      *reinterpret_cast<uint2 *>(r1 + i * kGroup) = make_uint2(m1.x & ~mask, m1.y & ~mask);
-      *reinterpret_cast<uint2 *>(r2 + i * kGroup) = make_uint2((m1.x & mask) | (((m2.x & mask) ^ mask) << 16),
-                                                               (m1.y & mask) | (((m2.y & mask) ^ mask) << 16));
-    }
-  }
-  __syncthreads();
-  // counts from above the piece, and how many entries reach a minimum that several do
-  for (int i = warp; i < len; i += nw) {
-    const int4 m = p.meta[i];
-    const int nx = m.y - m.z - m.x;
-    unsigned long long c[K];
-    int a1[K], a2[K];
-    bool tie = false;
+  if (!__any_sync(kAll, tie)) return;
+  // several entries: those after the first, up to the last that any lane has
+  lo = __reduce_min_sync(kAll, lo);
+  hi = __reduce_max_sync(kAll, hi);
+  for (int q0 = lo; q0 <= hi; q0 += 8) {
+    int2 w[8];
+    uint2 d[8];
 #pragma unroll
-    for (int k = 0; k < K; k++) {
-      const unsigned ar = k2[(k >> 1) * gs + i * kGroup + (k & 1)];
-      a1[k] = (int)(ar & 0xffff);
-      a2[k] = (int)(ar >> 16);
-      tie |= a1[k] != a2[k];
-      const int e = m.x + max(a1[k], 1) - 1;
-      c[k] = 0;
-      if (a1[k] == 0) c[k] = a.Uc[gu[k >> 1] + (size_t)p.sub[i].y * kGroup + (k & 1)];
-      else if (a1[k] <= nx) c[k] = (unsigned long long)(unsigned)a.eC[e] * a.S[gt[k >> 1] + (size_t)a.ex[e].x * kGroup + (k & 1)];
-    }
-    if (__any_sync(kAll, tie)) {
+    for (int q = 0; q < 8; q++) w[q] = __ldg(a.ex + e0 + min(q0 + q, hi) - 1);
 #pragma unroll
-      for (int k = 0; k < K; k++) {
-        const bool tk = a1[k] != a2[k];
-        if (!__any_sync(kAll, tk)) continue;
-        uint32_t *r1 = k1 + (k >> 1) * gs + (k & 1);
-        const unsigned dt = r1[i * kGroup];
-        int hits = a1[k] == 0;
-        unsigned long long cc = hits ? c[k] : 0;  // every entry above the piece that reaches the minimum
-        for (int e = m.x; e < m.x + nx; e += 8) {
-          int2 v[8];
-          unsigned d[8];
+    for (int q = 0; q < 8; q++) d[q] = *reinterpret_cast<const uint2 *>(a.D + gt + (size_t)w[q].x * kGroup);
 #pragma unroll
-          for (int q = 0; q < 8; q++) v[q] = __ldg(a.ex + min(e + q, m.x + nx - 1));
-#pragma unroll
-          for (int q = 0; q < 8; q++) d[q] = a.D[gt[k >> 1] + (size_t)v[q].x * kGroup + (k & 1)];
-#pragma unroll
-          for (int q = 0; q < 8; q++)
-            if (tk && e + q < m.x + nx && d[q] + ((unsigned)v[q].y & ~mask) == dt) {
-              hits++;
-              cc = count_of(a, cc + (unsigned long long)(unsigned)a.eC[e + q] * a.S[gt[k >> 1] + (size_t)v[q].x * kGroup + (k & 1)]);
-            }
-        }
-        for (int q = p.inoff[i]; q < p.inoff[i + 1]; q++)
-          hits += tk && r1[p.ine[q].x] + ((unsigned)p.ine[q].y & ~mask) == dt;
-        if (tk) {
-          c[k] = cc;
-          if (hits > 2) k2[(k >> 1) * gs + i * kGroup + (k & 1)] = (unsigned)a2[k] | ((unsigned)a1[k] << 16);
-        }
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < K; k++) sg[(k >> 1) * gs + i * kGroup + (k & 1)] = count_of(a, c[k]);
-  }
-  __syncthreads();
-  // counts from inside the piece, along it
-  if (warp < GB) {
-    uint32_t *r1 = k1 + warp * gs, *r2 = k2 + warp * gs, *rs = sg + warp * gs;
-    for (int i = 1; i < len; i++) {
-      const int4 m = p.meta[i];
-      const int nx = m.y - m.z - m.x, in0 = p.inoff[i] - 1 - nx;
-      const uint2 ar = *reinterpret_cast<uint2 *>(r2 + i * kGroup);
+    for (int q = 0; q < 8; q++)
 #pragma unroll
       for (int k = 0; k < 2; k++) {
-        const int a1 = (int)((k ? ar.y : ar.x) & 0xffff), a2 = (int)((k ? ar.y : ar.x) >> 16);
-        if (max(a1, a2) <= nx) continue;
-        unsigned long long c = rs[i * kGroup + k];
-        if (a1 <= a2) {
-          if (a1 > nx) c += (unsigned long long)(unsigned)p.ineC[in0 + a1] * rs[p.ine[in0 + a1].x + k];
-          if (a2 > nx && a1 != a2) c += (unsigned long long)(unsigned)p.ineC[in0 + a2] * rs[p.ine[in0 + a2].x + k];
-        } else {
-          const unsigned dt = r1[i * kGroup + k];
-          for (int q = p.inoff[i]; q < p.inoff[i + 1]; q++)
-            if (r1[p.ine[q].x + k] + ((unsigned)p.ine[q].y & ~mask) == dt)
-              c = count_of(a, c + (unsigned long long)(unsigned)p.ineC[q] * rs[p.ine[q].x + k]);
+        const int a1 = (int)(ar[k] & 0xffff), a2 = (int)(ar[k] >> 16);
+        if (q0 + q <= hi && a1 < q0 + q && q0 + q <= a2 && (k ? d[q].y : d[q].x) + ((unsigned)w[q].y & ~mask) == md[k]) {
+          const unsigned long long c =
+              cnt[k] + (unsigned long long)(unsigned)a.eC[e0 + q0 + q - 1] * a.S[gt + (size_t)w[q].x * kGroup + k];
+          over |= c > 0x7fffffffull;
+          cnt[k] = (uint32_t)c;
+          hits[k]++;
         }
-        rs[i * kGroup + k] = count_of(a, c);
       }
+  }
+}
+
+template <int PL>
+__global__ void __launch_bounds__(Wide<PL>::warps * 32) k_trunk_down(TreeArgs a, int piece0) {
+  constexpr int NW = Wide<PL>::warps;
+  __shared__ PieceShared<PL> p;
+  // per vertex and source: distance and argument (before its turn on the path: the two keys of the
+  // minimum above the piece), count (sign bit before its turn: more than two entries reach it)
+  __shared__ uint2 sd[PL * 32], sa[PL * 32], sc[PL * 32];
+  if (__syncthreads_or(wrapped(a))) return;
+  const int4 pc = a.piece[piece0 + blockIdx.x];
+  const int start = pc.x, len = pc.y - pc.x, g = blockIdx.y;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const unsigned mask = (1u << a.bits) - 1u;
+  uint2 *rd = sd + lane, *ra = sa + lane, *rc = sc + lane;
+  int s[2];
+  bool live[2];
+  lane_sources(a, g, lane, s, live);
+  const size_t gt = (size_t)g * a.NT * kGroup + 2 * lane, gu = (size_t)g * a.H * kGroup + 2 * lane;
+  load_piece<PL>(a, start, len, p);
+  __syncthreads();
+  unsigned over = 0;
+  for (int i = warp; i < len; i += NW) {
+    const int4 m = p.meta[i];
+    const int2 sub = p.sub[i];
+    const size_t u = gu + (size_t)sub.y * kGroup;
+    unsigned m1[2], m2[2], md[2], ar[2], hits[2];
+    uint32_t cnt[2];
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+      m1[k] = up_key(a, m.w <= s[k] && s[k] < sub.x, u + k);
+      m2[k] = m1[k] == kNoKey ? kNoKey : m1[k] ^ mask;
     }
+    scan_above(a, m.x, m.y - m.z, gt, mask, m1, m2);
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+      md[k] = m1[k] & ~mask;
+      ar[k] = (m1[k] & mask) | (((m2[k] & mask) ^ mask) << 16);
+    }
+    count_above(a, m.x, m.y - m.z - m.x, gt, u, mask, md, ar, cnt, hits, over);
+    rd[i * 32] = make_uint2(m1[0], m1[1]);
+    ra[i * 32] = make_uint2(m2[0], m2[1]);
+    rc[i * 32] = make_uint2(cnt[0] | (hits[0] > 2 ? 0x80000000u : 0u), cnt[1] | (hits[1] > 2 ? 0x80000000u : 0u));
   }
   __syncthreads();
-  for (int task = warp; task < len * GB; task += nw) {
-    const int w = task / len, i = task - w * len;
-    if (g0 + w >= a.ng) break;
-    const size_t o = ((size_t)(g0 + w) * a.NT + start + i) * kGroup + 2 * lane;
-    const int q = w * gs + i * kGroup;
-    *reinterpret_cast<uint2 *>(a.D + o) = *reinterpret_cast<uint2 *>(k1 + q);
-    *reinterpret_cast<uint2 *>(a.S + o) = *reinterpret_cast<uint2 *>(sg + q);
-    *reinterpret_cast<uint2 *>(a.arg + o) = *reinterpret_cast<uint2 *>(k2 + q);
+  if (warp == 0) {  // along the piece: entries inside it, in order
+    for (int i = 0; i < len; i++) {
+      const uint2 e1 = rd[i * 32], e2 = ra[i * 32], ec = rc[i * 32];
+      const unsigned x1[2] = {e1.x, e1.y}, x2[2] = {e2.x, e2.y};  // above the piece
+      unsigned m1[2] = {e1.x, e1.y}, m2[2] = {e2.x, e2.y};
+      const int b = p.inoff[i], e = p.inoff[i + 1];
+#pragma unroll 4
+      for (int q = b; q < e; q++) {
+        const int2 v = p.ine[q];
+        const uint2 d = rd[v.x >> 1];
+        const unsigned w0 = d.x + (unsigned)v.y, w1 = d.y + (unsigned)v.y;
+        m1[0] = min(m1[0], w0);
+        m2[0] = min(m2[0], w0 ^ mask);
+        m1[1] = min(m1[1], w1);
+        m2[1] = min(m2[1], w1 ^ mask);
+      }
+      const int4 m = p.meta[i];
+      const int nx = m.y - m.z - m.x;
+      unsigned ar[2];
+      uint32_t cnt[2] = {ec.x & 0x7fffffffu, ec.y & 0x7fffffffu};
+      bool tie = false;
+#pragma unroll
+      for (int k = 0; k < 2; k++) {
+        const int a1 = (int)(m1[k] & mask);
+        ar[k] = (unsigned)a1 | ((unsigned)a1 << 16);
+        tie |= (m1[k] ^ m2[k]) != mask;
+        if (a1 > nx) {
+          const int q = b + a1 - 1 - nx;
+          const uint2 c = rc[p.ine[q].x >> 1];
+          const unsigned long long z = (unsigned long long)(unsigned)p.ineC[q] * (k ? c.y : c.x);
+          over |= z > 0x7fffffffull;
+          cnt[k] = (uint32_t)z;
+        }
+      }
+      if (__any_sync(kAll, tie)) {  // several entries: their counts summed
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+          if ((m1[k] ^ m2[k]) == mask) continue;
+          const unsigned dt = m1[k] & ~mask;
+          const uint32_t c0 = (k ? ec.y : ec.x);
+          int hits = 0;
+          unsigned long long z = 0;
+          if ((x1[k] & ~mask) == dt) {  // some above the piece
+            hits = (x1[k] ^ x2[k]) == mask ? 1 : c0 >> 31 ? 3 : 2;
+            z = c0 & 0x7fffffffu;
+          }
+          for (int q = b; q < e; q++) {
+            const int2 v = p.ine[q];
+            const uint2 d = rd[v.x >> 1];
+            if ((k ? d.y : d.x) + ((unsigned)v.y & ~mask) != dt) continue;
+            const uint2 c = rc[v.x >> 1];
+            z += (unsigned long long)(unsigned)p.ineC[q] * (k ? c.y : c.x);
+            if (z > 0x7fffffffull) {
+              over = 1;
+              z = 1;
+            }
+            hits++;
+          }
+          cnt[k] = (uint32_t)z;
+          const unsigned lo = m1[k] & mask, hi = (m2[k] & mask) ^ mask;
+          ar[k] = hits > 2 ? hi | (lo << 16) : lo | (hi << 16);
+        }
+      }
+      rd[i * 32] = make_uint2(m1[0] & ~mask, m1[1] & ~mask);
+      ra[i * 32] = make_uint2(ar[0], ar[1]);
+      rc[i * 32] = make_uint2(cnt[0], cnt[1]);
+    }
+  }
+  if (over) *a.wrap = 1;
+  __syncthreads();
+  for (int i = warp; i < len; i += NW) {
+    const size_t o = gt + (size_t)(start + i) * kGroup;
+    *reinterpret_cast<uint2 *>(a.D + o) = rd[i * 32];
+    *reinterpret_cast<uint2 *>(a.S + o) = rc[i * 32];
+    *reinterpret_cast<uint2 *>(a.arg + o) = ra[i * 32];
     *reinterpret_cast<double2 *>(a.J + o) = make_double2(0.0, 0.0);
   }
 }
 
-// ------------------------------------------------------------------------------- trunk up
-template <int GB>
-__global__ void __launch_bounds__(512) k_trunk_up(TreeArgs a, int piece0, int pl) {
-  extern __shared__ double sm_tu[];
-  __shared__ PieceShared p;
-  constexpr int K = 2 * GB;
-  const unsigned mask = (1u << a.bits) - 1u;
+// What a trunk vertex does with its flow beyond its piece: the seed of its U row, flow to the entries
+// above the piece, and the flow through each of its shortcuts.  one: its argument where it is the
+// only one, xi that entry's trunk index.
+__device__ __forceinline__ void hand_up(const TreeArgs &a, const int4 m, const int2 sub, size_t gt, size_t gu, unsigned mask,
+                                        const int (&s)[2], const int (&si)[2], const bool (&live)[2], const double (&f)[2],
+                                        const unsigned (&ar)[2], int (&one)[2], const int (&xi)[2], size_t own) {
+  const int nx = m.y - m.z - m.x;
+  bool tie = false;
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    const int a1 = (int)(ar[k] & 0xffff), a2 = (int)(ar[k] >> 16);
+    tie |= a1 != a2;
+    if (live[k] && m.w <= s[k] && s[k] < sub.x) {
+      const size_t u = gu + (size_t)sub.y * kGroup + k;
+      a.seed[u] = min(a1, a2) != 0 ? 0.0 : a1 == a2 ? f[k] : f[k] * share(1, a.Uc[u], a.S[own + k]);
+    }
+    if (one[k] > 0 && one[k] <= nx) atomicAdd(a.J + gt + (size_t)xi[k] * kGroup + k, f[k]);
+    if (xi[k] == si[k]) {  // flow into the lane's own source counts apart
+      atomicAdd(a.Bs + m.x + one[k] - 1, f[k]);
+      one[k] = 0;
+    }
+  }
+  add_flows<2>(a, m.x, one, f);
+  if (!__any_sync(kAll, tie)) return;
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    const int a1 = (int)(ar[k] & 0xffff), a2 = (int)(ar[k] >> 16);
+    if (a1 == a2) continue;
+    const uint32_t st = a.S[own + k];
+    auto use = [&](int idx) {
+      const int e = m.x + idx - 1, x = a.ex[e].x;
+      const double w = f[k] * share(a.eC[e], a.S[gt + (size_t)x * kGroup + k], st);
+      if (idx <= nx) atomicAdd(a.J + gt + (size_t)x * kGroup + k, w);
+      atomicAdd((x == si[k] ? a.Bs : a.Bd) + e, w);
+    };
+    if (a1 < a2) {
+      if (a1 > 0) use(a1);
+      use(a2);
+    } else {  // more than two entries
+      const unsigned dt = a.D[own + k];
+      for (int e = m.x; e < m.y; e++) {
+        const int2 x = a.ex[e];
+        if (a.D[gt + (size_t)x.x * kGroup + k] + ((unsigned)x.y & ~mask) == dt) use(e - m.x + 1);
+      }
+    }
+  }
+}
+
+template <int PL>
+__global__ void __launch_bounds__(Wide<PL>::warps * 32) k_trunk_up(TreeArgs a, int piece0) {
+  constexpr int NW = Wide<PL>::warps;
+  __shared__ PieceShared<PL> p;
+  __shared__ double2 sf[PL * 32];
+  __shared__ uint2 sa[PL * 32], ss[PL * 32];
   if (__syncthreads_or(wrapped(a))) return;
   const int4 pc = a.piece[piece0 + blockIdx.x];
-  const int start = pc.x, len = pc.y - pc.x;
-  const int g0 = blockIdx.y * GB;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  const int gs = pl * kGroup;
-  double *sf = sm_tu + 2 * lane;  // flow of a vertex: delta + 1 (delta for the source itself)
-  uint32_t *sa = reinterpret_cast<uint32_t *>(sm_tu + GB * gs) + 2 * lane;
-  int s[K], si[K];
-  bool live[K];
-  size_t gt[GB], gu[GB];
+  const int start = pc.x, len = pc.y - pc.x, g = blockIdx.y;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const unsigned mask = (1u << a.bits) - 1u;
+  double *rf = &sf[lane].x;  // flow of a vertex: delta + 1 (delta for the source itself)
+  uint32_t *ra = &sa[lane].x, *rs = &ss[lane].x;
+  int s[2], si[2];
+  bool live[2];
+  lane_sources(a, g, lane, s, live);
 #pragma unroll
-  for (int w = 0; w < GB; w++) {
-    const int g = min(g0 + w, a.ng - 1);
-    bool lw[2];
-    int sw[2];
-    lane_sources(a, g, lane, sw, lw);
-#pragma unroll
-    for (int k = 0; k < 2; k++) {
-      s[2 * w + k] = sw[k];
-      live[2 * w + k] = lw[k] && g0 + w < a.ng;
-      si[2 * w + k] = a.tidx_of[sw[k]];
-    }
-    gt[w] = (size_t)g * a.NT * kGroup + 2 * lane;
-    gu[w] = (size_t)g * a.H * kGroup + 2 * lane;
-  }
-  load_piece(a, start, len, p);
+  for (int k = 0; k < 2; k++) si[k] = a.tidx_of[s[k]];
+  const size_t gt = (size_t)g * a.NT * kGroup + 2 * lane, gu = (size_t)g * a.H * kGroup + 2 * lane;
+  load_piece<PL>(a, start, len, p);
   __syncthreads();
-  for (int i = warp; i < len; i += nw) {
+  for (int i = warp; i < len; i += NW) {
     const int t = p.meta[i].w;
-#pragma unroll
-    for (int w = 0; w < GB; w++) {
-      const size_t o = gt[w] + (size_t)(start + i) * kGroup;
-      const double2 j = __ldcg(reinterpret_cast<const double2 *>(a.J + o));
-      const uint2 ar = *reinterpret_cast<const uint2 *>(a.arg + o);
-      const bool l0 = live[2 * w], l1 = live[2 * w + 1];
-      // a lane without a source has no flow and no argument
-      *reinterpret_cast<double2 *>(sf + w * gs + i * kGroup) =
-          make_double2(l0 ? j.x + (t != s[2 * w] ? 1.0 : 0.0) : 0.0, l1 ? j.y + (t != s[2 * w + 1] ? 1.0 : 0.0) : 0.0);
-      *reinterpret_cast<uint2 *>(sa + w * gs + i * kGroup) = make_uint2(l0 ? ar.x : 0u, l1 ? ar.y : 0u);
-    }
+    const size_t o = gt + (size_t)(start + i) * kGroup;
+    const double2 j = __ldcg(reinterpret_cast<const double2 *>(a.J + o));
+    const uint2 x = *reinterpret_cast<const uint2 *>(a.arg + o), y = *reinterpret_cast<const uint2 *>(a.S + o);
+    // a lane without a source has no flow and no argument
+    *reinterpret_cast<double2 *>(rf + i * kGroup) =
+        make_double2(live[0] ? j.x + (t != s[0] ? 1.0 : 0.0) : 0.0, live[1] ? j.y + (t != s[1] ? 1.0 : 0.0) : 0.0);
+    *reinterpret_cast<uint2 *>(ra + i * kGroup) = make_uint2(live[0] ? x.x : 0u, live[1] ? x.y : 0u);
+    *reinterpret_cast<uint2 *>(rs + i * kGroup) = y;
   }
   __syncthreads();
-  // what is handed on inside the piece, a warp per group, deepest vertex first
-  if (warp < GB) {
-    double *rf = sf + warp * gs;
-    const uint32_t *ra = sa + warp * gs;
+  if (warp == 0) {  // what is handed on inside the piece, deepest vertex first
     for (int i = len - 1; i > 0; i--) {
       const int4 m = p.meta[i];
+      if (m.z == 0) continue;
       const int nx = m.y - m.z - m.x, in0 = p.inoff[i] - 1 - nx;
       const uint2 ar = *reinterpret_cast<const uint2 *>(ra + i * kGroup);
       const double2 f2 = *reinterpret_cast<const double2 *>(rf + i * kGroup);
@@ -736,81 +791,208 @@ __global__ void __launch_bounds__(512) k_trunk_up(TreeArgs a, int piece0, int pl
         if (max(a1, a2) <= nx) continue;
         if (a1 == a2) {
           rf[p.ine[in0 + a1].x + k] += f;
-        } else {
-          const size_t gp = ((size_t)(g0 + warp) * a.NT + start) * kGroup + 2 * lane + k;
-          const uint32_t st = a.S[gp + (size_t)i * kGroup];
+        } else if (a1 < a2) {
+          const uint32_t st = rs[i * kGroup + k];
+          const int x2 = p.ine[in0 + a2].x + k;
+          if (a1 > nx) {
+            const int x1 = p.ine[in0 + a1].x + k;
+            rf[x1] += share(p.ineC[in0 + a1], rs[x1], st) * f;
+          }
+          rf[x2] += share(p.ineC[in0 + a2], rs[x2], st) * f;
+        } else {  // more than two entries
+          const size_t gp = gt + (size_t)start * kGroup + k;
           const unsigned dt = a.D[gp + (size_t)i * kGroup];
           for (int q = p.inoff[i]; q < p.inoff[i + 1]; q++) {
             const int x = p.ine[q].x;
-            const bool hit = a1 < a2 ? q == in0 + a1 || q == in0 + a2 : a.D[gp + x] + ((unsigned)p.ine[q].y & ~mask) == dt;
-            if (hit) rf[x + k] += share(p.ineC[q], a.S[gp + x], st) * f;
+            if (a.D[gp + x] + ((unsigned)p.ine[q].y & ~mask) == dt)
+              rf[x + k] += share(p.ineC[q], rs[x + k], rs[i * kGroup + k]) * f;
           }
         }
       }
     }
   }
   __syncthreads();
-  // everything else of a vertex, a warp with all the CTA's sources
-  for (int i = warp; i < len; i += nw) {
+  for (int i = warp; i < len; i += NW) {  // everything else, a warp per vertex
     const int4 m = p.meta[i];
-    const int2 sub = p.sub[i];
-    const int nx = m.y - m.z - m.x;
-    int a1[K], a2[K], one[K];
-    double f[K];
-    bool tie = false;
+    const uint2 x = *reinterpret_cast<const uint2 *>(ra + i * kGroup);
+    const double2 f2 = *reinterpret_cast<const double2 *>(rf + i * kGroup);
+    const unsigned ar[2] = {x.x, x.y};
+    const double f[2] = {f2.x, f2.y};
+    int one[2], xi[2];
 #pragma unroll
-    for (int k = 0; k < K; k++) {
-      const unsigned ar = sa[(k >> 1) * gs + i * kGroup + (k & 1)];
-      a1[k] = (int)(ar & 0xffff);
-      a2[k] = (int)(ar >> 16);
-      f[k] = sf[(k >> 1) * gs + i * kGroup + (k & 1)];
-      tie |= a1[k] != a2[k];
-      one[k] = a1[k] == a2[k] ? a1[k] : 0;
+    for (int k = 0; k < 2; k++) {
+      one[k] = (ar[k] & 0xffff) == (ar[k] >> 16) ? (int)(ar[k] & 0xffff) : 0;
+      xi[k] = one[k] > 0 ? a.ex[m.x + one[k] - 1].x : INT_MIN;
+    }
+    hand_up(a, m, p.sub[i], gt, gu, mask, s, si, live, f, ar, one, xi, gt + (size_t)(start + i) * kGroup);
+  }
+}
+
+// ------------------------------------------------------------------------------- trunk, narrow levels
+// Levels with few pieces wait for the longest one, so a CTA of 32 warps takes a piece, a warp per
+// vertex.  The path is followed vertex by vertex: a vertex's warp publishes its distances and counts,
+// and the warps of the vertices below offer them to their running minimum, arguments and count in
+// registers.  (One warp walking the path alone takes 23k cycles for the distances and 16k for the
+// counts of a full piece.)
+struct PieceTable {
+  unsigned win[kPieceLen][kPieceLen + 1];  // key of the edge (vertex, earlier vertex), or absent
+  int cin[kPieceLen][kPieceLen + 1];       // its count
+};
+
+__device__ __forceinline__ void load_table(const TreeArgs &a, int start, int len, PieceTable &p) {
+  const int i = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (i >= len) return;
+  const int4 m = a.tmeta[start + i];
+  p.win[i][lane] = a.absent;
+  __syncwarp();
+  if (lane < m.z) {  // at most 31 edges inside the piece
+    const int2 v = a.ex[m.y - m.z + lane];
+    p.win[i][v.x - start] = (unsigned)v.y;
+    p.cin[i][v.x - start] = a.eC[m.y - m.z + lane];
+  }
+}
+
+__global__ void __launch_bounds__(kPieceLen * 32) k_trunk_down_narrow(TreeArgs a, int piece0) {
+  __shared__ PieceTable p;
+  __shared__ uint2 row_d[2][32], row_c[2][32];
+  if (__syncthreads_or(wrapped(a))) return;
+  const int4 pc = a.piece[piece0 + blockIdx.x];
+  const int start = pc.x, len = pc.y - pc.x, g = blockIdx.y;
+  const int i = threadIdx.x >> 5, lane = threadIdx.x & 31;  // this warp's vertex
+  const unsigned mask = (1u << a.bits) - 1u;
+  const size_t gt = (size_t)g * a.NT * kGroup + 2 * lane;
+  load_table(a, start, len, p);
+  unsigned md[2] = {}, ar[2] = {}, hits[2] = {}, over = 0;
+  uint32_t cnt[2] = {};
+  if (i < len) {
+    int s[2];
+    bool live[2];
+    lane_sources(a, g, lane, s, live);
+    const int4 m = a.tmeta[start + i];
+    const int2 sub = a.tsub[start + i];
+    const size_t u = ((size_t)g * a.H + sub.y) * kGroup + 2 * lane;
+    unsigned m1[2], m2[2];
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+      m1[k] = up_key(a, m.w <= s[k] && s[k] < sub.x, u + k);
+      m2[k] = m1[k] == kNoKey ? kNoKey : m1[k] ^ mask;
+    }
+    scan_above(a, m.x, m.y - m.z, gt, mask, m1, m2);
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+      md[k] = m1[k] & ~mask;
+      ar[k] = (m1[k] & mask) | (((m2[k] & mask) ^ mask) << 16);
+    }
+    count_above(a, m.x, m.y - m.z - m.x, gt, u, mask, md, ar, cnt, hits, over);
+  }
+  for (int t = 0; t < len; t++) {
+    if (t == i) {
+      row_d[t & 1][lane] = make_uint2(md[0], md[1]);
+      row_c[t & 1][lane] = make_uint2(cnt[0], cnt[1]);
+    }
+    __syncthreads();  // (also the tables, the first time)
+    if (t >= i || i >= len) continue;
+    const unsigned key = p.win[i][t];
+    if (key == a.absent) continue;
+    const uint2 d2 = row_d[t & 1][lane], c2 = row_c[t & 1][lane];
+    const unsigned idx = key & mask;
+    const int C = p.cin[i][t];
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+      const unsigned d = (k ? d2.y : d2.x) + (key & ~mask);
+      if (d > md[k]) continue;
+      if (d < md[k]) {
+        md[k] = d;
+        ar[k] = idx;
+        hits[k] = 0;
+        cnt[k] = 0;
+      }
+      const unsigned long long c = (unsigned long long)(unsigned)C * (k ? c2.y : c2.x) + cnt[k];
+      over |= c > 0x7fffffffull;
+      cnt[k] = (uint32_t)c;
+      ar[k] = (ar[k] & 0xffff) | (idx << 16);
+      hits[k]++;
+    }
+  }
+  if (over) *a.wrap = 1;
+  if (i >= len) return;
+#pragma unroll
+  for (int k = 0; k < 2; k++)
+    if (hits[k] > 2) ar[k] = (ar[k] >> 16) | (ar[k] << 16);
+  const size_t o = gt + (size_t)(start + i) * kGroup;
+  *reinterpret_cast<uint2 *>(a.D + o) = make_uint2(md[0], md[1]);
+  *reinterpret_cast<uint2 *>(a.S + o) = make_uint2(cnt[0], cnt[1]);
+  *reinterpret_cast<uint2 *>(a.arg + o) = make_uint2(ar[0], ar[1]);
+  *reinterpret_cast<double2 *>(a.J + o) = make_double2(0.0, 0.0);
+}
+
+// The same, deepest vertex first: a vertex's warp publishes its flow and arguments, and the warps of
+// the vertices above take their share of it.
+__global__ void __launch_bounds__(kPieceLen * 32) k_trunk_up_narrow(TreeArgs a, int piece0) {
+  __shared__ PieceTable p;
+  __shared__ double2 row_f[2][32];
+  __shared__ uint2 row_a[2][32], row_s[2][32], row_d[2][32];
+  if (__syncthreads_or(wrapped(a))) return;
+  const int4 pc = a.piece[piece0 + blockIdx.x];
+  const int start = pc.x, len = pc.y - pc.x, g = blockIdx.y;
+  const int i = threadIdx.x >> 5, lane = threadIdx.x & 31;  // this warp's vertex
+  const unsigned mask = (1u << a.bits) - 1u;
+  const size_t gt = (size_t)g * a.NT * kGroup + 2 * lane, gu = (size_t)g * a.H * kGroup + 2 * lane;
+  const size_t own = gt + (size_t)(start + i) * kGroup;
+  int4 m = make_int4(0, 0, 0, 0);
+  int s[2], si[2], one[2], xi[2];
+  bool live[2];
+  double f[2] = {};
+  unsigned ar[2] = {};
+  uint2 st = make_uint2(0, 0), dt = st;
+  lane_sources(a, g, lane, s, live);
+  if (i < len) {
+    const double2 j = __ldcg(reinterpret_cast<const double2 *>(a.J + own));
+    const uint2 x = *reinterpret_cast<const uint2 *>(a.arg + own);
+    st = *reinterpret_cast<const uint2 *>(a.S + own);
+    dt = *reinterpret_cast<const uint2 *>(a.D + own);
+    m = a.tmeta[start + i];
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+      si[k] = a.tidx_of[s[k]];
+      if (!live[k]) continue;  // a lane without a source has no flow and no argument
+      ar[k] = k ? x.y : x.x;
+      f[k] = (k ? j.y : j.x) + (m.w != s[k] ? 1.0 : 0.0);
     }
 #pragma unroll
-    for (int k = 0; k < K; k++)
-      if (live[k] && m.w <= s[k] && s[k] < sub.x) {
-        const size_t u = gu[k >> 1] + (size_t)sub.y * kGroup + (k & 1);
-        const int lo = min(a1[k], a2[k]);
-        a.seed[u] = lo != 0 ? 0.0 : a1[k] == a2[k] ? f[k] : f[k] * share(1, a.Uc[u], a.S[gt[k >> 1] + (size_t)(start + i) * kGroup + (k & 1)]);
-      }
-    int xi[K];
-#pragma unroll
-    for (int k = 0; k < K; k++) xi[k] = one[k] > 0 ? a.ex[m.x + one[k] - 1].x : INT_MIN;
-#pragma unroll
-    for (int k = 0; k < K; k++) {
-      if (one[k] > 0 && one[k] <= nx) atomicAdd(a.J + gt[k >> 1] + (size_t)xi[k] * kGroup + (k & 1), f[k]);
-      if (xi[k] == si[k]) {  // flow into the lane's own source counts apart
-        atomicAdd(a.Bs + m.x + one[k] - 1, f[k]);
-        one[k] = 0;
-      }
+    for (int k = 0; k < 2; k++) {
+      one[k] = (ar[k] & 0xffff) == (ar[k] >> 16) ? (int)(ar[k] & 0xffff) : 0;
+      xi[k] = one[k] > 0 ? a.ex[m.x + one[k] - 1].x : INT_MIN;
     }
-    add_flows<K>(a, m.x, one, f);
-    if (__any_sync(kAll, tie)) {
+  }
+  load_table(a, start, len, p);
+  for (int t = len - 1; t > 0; t--) {
+    if (t == i) {
+      row_f[t & 1][lane] = make_double2(f[0], f[1]);
+      row_a[t & 1][lane] = make_uint2(ar[0], ar[1]);
+      row_s[t & 1][lane] = st;
+      row_d[t & 1][lane] = dt;
+    }
+    __syncthreads();  // (also the tables, the first time)
+    if (i >= t) continue;
+    const unsigned key = p.win[t][i];
+    if (key == a.absent) continue;
+    const uint2 a2 = row_a[t & 1][lane];
+    const double2 f2 = row_f[t & 1][lane];
+    const unsigned idx = key & mask;
 #pragma unroll
-      for (int k = 0; k < K; k++) {
-        if (a1[k] == a2[k]) continue;
-        const size_t gk = gt[k >> 1] + (k & 1);
-        const uint32_t st = a.S[gk + (size_t)(start + i) * kGroup];
-        const unsigned dt = a.D[gk + (size_t)(start + i) * kGroup];
-        auto use = [&](int idx) {
-          const int e = m.x + idx - 1, x = a.ex[e].x;
-          const double w = f[k] * share(a.eC[e], a.S[gk + (size_t)x * kGroup], st);
-          if (idx <= nx) atomicAdd(a.J + gk + (size_t)x * kGroup, w);
-          atomicAdd((x == si[k] ? a.Bs : a.Bd) + e, w);
-        };
-        if (a1[k] < a2[k]) {
-          if (a1[k] > 0) use(a1[k]);
-          use(a2[k]);
-        } else {  // more than two entries
-          for (int e = m.x; e < m.y; e++) {
-            const int2 v = a.ex[e];
-            if (a.D[gk + (size_t)v.x * kGroup] + ((unsigned)v.y & ~mask) == dt) use(e - m.x + 1);
-          }
-        }
+    for (int k = 0; k < 2; k++) {
+      const unsigned x1 = (k ? a2.y : a2.x) & 0xffff, x2 = (k ? a2.y : a2.x) >> 16;
+      if (x1 == x2) {
+        if (x1 == idx) f[k] += k ? f2.y : f2.x;
+      } else if (x1 > x2 || x1 == idx || x2 == idx) {
+        const uint2 s2 = row_s[t & 1][lane], d2 = row_d[t & 1][lane];
+        if (x1 < x2 || (k ? dt.y : dt.x) + (key & ~mask) == (k ? d2.y : d2.x))
+          f[k] += (k ? f2.y : f2.x) * share(p.cin[t][i], k ? st.y : st.x, k ? s2.y : s2.x);
       }
     }
   }
+  if (i < len) hand_up(a, m, a.tsub[start + i], gt, gu, mask, s, si, live, f, ar, one, xi, own);
 }
 
 // ------------------------------------------------------------------------------- bottoms
@@ -822,12 +1004,17 @@ __global__ void __launch_bounds__(512) k_trunk_up(TreeArgs a, int piece0, int pl
 // to 1.3 different entries per vertex and warp): that entry's flow stays in the finished row and is
 // summed after the pass, eight rows at a time, instead of by a warp-wide sum per vertex.
 //
+// A vertex without descendants (44 % of them) that hands everything to one entry in all lanes is done
+// at once on the way down: its flow is 1 per source, and nobody reads its row.
+//
 // The pass is bound by instruction issue, so shared memory is addressed by 32-bit offsets (ld.shared
 // / st.shared); a row's block holds delta (f64), distance, count and argument of the warp's sources.
 constexpr int kTieCode = 0xff, kSkipCode = 0xfe;  // arguments that are no row: a tie, a lane without a source
 constexpr int kBottomPairs = (kBottomEdges + kBottomRows) / 2 + 1;
 constexpr int kBottomWarps = 2;
 constexpr int kLeadFull = 1 << 16;  // deferred sum: every lane, the rows' delta + 1 each
+constexpr int kManyCounts = INT_MIN, kLeaf = 1 << 30, kDepthBits = kLeaf - 1;  // in a vertex's fourth word
+constexpr int kAhead = 8;           // separator rows of the next group loaded during the way up
 
 struct RowLayout {  // bytes
   static constexpr int D = 512, S = 768, G = 1024, lead = 1088, size = 1104;
@@ -874,13 +1061,14 @@ __device__ __forceinline__ void code_store(uint32_t p, unsigned v) {
   asm volatile("st.shared.u16 [%0], %1;" ::"r"(p), "h"((unsigned short)v) : "memory");
 }
 
-__global__ void __launch_bounds__(kBottomWarps * 32) k_bottom(TreeArgs a, int first, int rows, int gpc, unsigned absent) {
+__global__ void __launch_bounds__(kBottomWarps * 32) k_bottom(TreeArgs a, int first, int rows, int gpc) {
   extern __shared__ int4 sm_b[];
   using R = RowLayout;
   constexpr int SPL = 2;
   __shared__ int4 ep[kBottomPairs];           // two edges: (x row offset, key) twice
   __shared__ int2 er[kBottomEdges];           // an edge: (x row + 1, count)
-  __shared__ int4 vt[kBottomRows + 1];        // a vertex: (address of its first pair, end, first edge | edges << 16, depth - 1 | counts above 1 << 31)
+  __shared__ int4 vt[kBottomRows + 1];        // a vertex: (address of its first pair, end, first edge | edges << 16, depth - 1 | kLeaf | kManyCounts)
+  __shared__ uint8_t leaf_units[kBottomWarps][kBottomEdges];  // groups (at most 64) whose leaf handed everything to the edge
   __shared__ int vs[kBottomRows], sep[kBottomRows];  // subtree end, trunk index
   __shared__ uint8_t emap[kBottomRows][kBottomRows + 4];  // edge of (vertex, x row)
   if (__syncthreads_or(wrapped(a))) return;
@@ -904,13 +1092,14 @@ __global__ void __launch_bounds__(kBottomWarps * 32) k_bottom(TreeArgs a, int fi
   }
   for (int i = threadIdx.x; i < m; i += blockDim.x) vs[i] = a.send[r + i];
   for (int i = threadIdx.x; i < b; i += blockDim.x) sep[i] = a.etr[ebase + i];
+  for (int i = threadIdx.x; i < kBottomWarps * kBottomEdges; i += blockDim.x) (&leaf_units[0][0])[i] = 0;
   __syncthreads();
   for (int t = warp; t < m; t += nw) {
     const int4 v = vt[t];
     const int e0 = v.z & 0xffff, k = v.z >> 16;
     bool many = false;
     if (lane < max(2, (k + 1) & ~1)) {
-      const int2 x = lane < k ? a.ex[ebase + e0 + lane] : make_int2(0, (int)absent);
+      const int2 x = lane < k ? a.ex[ebase + e0 + lane] : make_int2(0, (int)a.absent);
       reinterpret_cast<int2 *>(ep + (((uint32_t)v.x - ep0) >> 4))[lane] = make_int2(x.x * R::size, x.y);
       if (lane < k) {
         const int c = a.eC[ebase + e0 + lane];
@@ -919,29 +1108,61 @@ __global__ void __launch_bounds__(kBottomWarps * 32) k_bottom(TreeArgs a, int fi
         emap[t][x.x] = (uint8_t)(e0 + lane);
       }
     }
-    if (__any_sync(kAll, many) && lane == 0) vt[t].w |= INT_MIN;
+    many = __any_sync(kAll, many);
+    if (lane == 0) vt[t].w |= (many ? kManyCounts : 0) | (vs[t] == r + t + 1 ? kLeaf : 0);
   }
   __syncthreads();
   const uint32_t base = (uint32_t)__cvta_generic_to_shared(sm_b) + (uint32_t)warp * (uint32_t)rows * R::size;
   const uint32_t bJ = base + lane * 8 * SPL, bD = base + R::D + lane * 4 * SPL, bG = base + R::G + lane * SPL;
   const unsigned mask = (1u << a.bits) - 1u;
   const int gend = min(a.ng, ((int)blockIdx.y + 1) * gpc);
-  for (int g = blockIdx.y * gpc + warp; g < gend; g += nw) {
+  // the next group's sources and first separator rows
+  int ns[SPL], nsi[SPL];
+  bool nlive[SPL];
+  uint2 nd[kAhead], nc[kAhead];
+  auto load_ahead = [&](int g) {
+    lane_sources(a, g, lane, ns, nlive);
+    const size_t gt = (size_t)g * a.NT * kGroup + 2 * lane;
+#pragma unroll
+    for (int q = 0; q < kAhead; q++)
+      if (q < b) {
+        nd[q] = __ldg(reinterpret_cast<const uint2 *>(a.D + gt + (size_t)sep[q] * kGroup));
+        nc[q] = __ldg(reinterpret_cast<const uint2 *>(a.S + gt + (size_t)sep[q] * kGroup));
+      }
+#pragma unroll
+    for (int k = 0; k < SPL; k++) nsi[k] = a.tidx_of[ns[k]];
+  };
+  const int gfirst = blockIdx.y * gpc + warp;
+  if (gfirst < gend) load_ahead(gfirst);
+  for (int g = gfirst; g < gend; g += nw) {
     int s[SPL], srow[SPL], si[SPL];
     bool live[SPL];
-    lane_sources(a, g, lane, s, live);
     const size_t gt = (size_t)g * a.NT * kGroup + 2 * lane, gu = (size_t)g * a.H * kGroup + 2 * lane;
     bool in_any = false, odd = false;
 #pragma unroll
     for (int k = 0; k < SPL; k++) {
+      s[k] = ns[k];
+      si[k] = nsi[k];
+      live[k] = nlive[k];
       srow[k] = r <= s[k] && s[k] < r + m ? b + s[k] - r : -1;  // the row of this lane's own source
       in_any |= srow[k] >= 0;
-      si[k] = a.tidx_of[s[k]];
     }
     const double zero[SPL] = {};
     const uint32_t none[SPL] = {};
     if (b == 0) row_store(bD, none);  // the whole tree: an absent entry of its root reads this row
-    for (int i = 0; i < b; i += 4) {  // the separator's rows, four loads of each in flight
+#pragma unroll
+    for (int q = 0; q < kAhead; q++)
+      if (q < b) {
+        const uint32_t d[SPL] = {nd[q].x, nd[q].y}, c[SPL] = {nc[q].x, nc[q].y};
+        row_store(bD + q * R::size, d);
+        row_store(bD + (R::S - R::D) + q * R::size, c);
+        row_store(bJ + q * R::size, zero);
+        const int sp = sep[q];
+#pragma unroll
+        for (int k = 0; k < SPL; k++)
+          if (sp == si[k]) srow[k] = q;
+      }
+    for (int i = kAhead; i < b; i += 4) {  // the separator's other rows, four loads of each in flight
       uint32_t d[4][SPL], c[4][SPL];
       int sp[4];
 #pragma unroll
@@ -969,7 +1190,7 @@ __global__ void __launch_bounds__(kBottomWarps * 32) k_bottom(TreeArgs a, int fi
     for (int k = 0; k < SPL; k++) odd |= srow[k] >= 0 || !live[k];
     // special: some lane's source lies among these rows, or lanes without a source
     const bool inside = __any_sync(kAll, in_any), special = __any_sync(kAll, odd);
-    unsigned over = 0;
+    unsigned over = 0, pending = m == 32 ? kAll : (1u << m) - 1u;  // vertices of the way up
     uint32_t off = b * R::size;  // of the current row
     int4 v = lds128(vt0), e = lds128(v.x);
     for (int t = 0; t < m; t++, off += R::size) {
@@ -981,7 +1202,7 @@ __global__ void __launch_bounds__(kBottomWarps * 32) k_bottom(TreeArgs a, int fi
         const int se = vs[t];
 #pragma unroll
         for (int k = 0; k < SPL; k++) {
-          m1[k] = up_key(a, r + t <= s[k] && s[k] < se, gu + (size_t)(v.w & INT_MAX) * kGroup + k);
+          m1[k] = up_key(a, r + t <= s[k] && s[k] < se, gu + (size_t)(v.w & kDepthBits) * kGroup + k);
           m2[k] = m1[k] == kNoKey ? kNoKey : m1[k] ^ mask;
         }
       }
@@ -1001,6 +1222,26 @@ __global__ void __launch_bounds__(kBottomWarps * 32) k_bottom(TreeArgs a, int fi
         }
       } while (pe < (uint32_t)v.y);
       e = lds128(vn.x);
+      if ((v.w & kLeaf) && !special) {
+        const unsigned x0 = m1[0] & mask;  // one entry for the lane's two sources, and for all lanes?
+        int all = 0;
+        __match_all_sync(kAll, ((m1[0] ^ m2[0]) == mask) & ((m1[1] ^ m2[1]) == mask) & ((m1[1] & mask) == x0) ? x0 : 0x100u + lane, &all);
+        if (all) {
+          double j[SPL];
+          const uint32_t xo = bJ + (x0 - 1) * R::size;
+          row_load(xo, j);
+#pragma unroll
+          for (int k = 0; k < SPL; k++) j[k] += 1.0;
+          row_store(xo, j);
+          uint8_t *lu = &leaf_units[warp][emap[t][x0 - 1]];
+          const uint8_t units = *lu + 1;
+          __syncwarp();
+          *lu = units;
+          pending &= ~(1u << t);
+          v = vn;
+          continue;
+        }
+      }
       unsigned x1[SPL];
       uint32_t c[SPL], dt[SPL];
       unsigned again = 0;  // several entries reach the minimum
@@ -1014,7 +1255,7 @@ __global__ void __launch_bounds__(kBottomWarps * 32) k_bottom(TreeArgs a, int fi
       if (inside)
 #pragma unroll
         for (int k = 0; k < SPL; k++)
-          if (x1[k] == 0) c[k] = a.Uc[gu + (size_t)(v.w & INT_MAX) * kGroup + k];
+          if (x1[k] == 0) c[k] = a.Uc[gu + (size_t)(v.w & kDepthBits) * kGroup + k];
       if (__any_sync(kAll, (again != 0) | (v.w < 0))) {  // or counts above 1: the edges once more
 #pragma unroll
         for (int k = 0; k < SPL; k++) {
@@ -1045,8 +1286,12 @@ __global__ void __launch_bounds__(kBottomWarps * 32) k_bottom(TreeArgs a, int fi
       v = vn;
     }
     if (over) *a.wrap = 1;
-    for (int t = m - 1; t >= 0; t--) {
-      off -= R::size;
+    if (g + nw < gend) load_ahead(g + nw);
+    const unsigned up = pending;
+    while (pending) {
+      const int t = 31 - __clz(pending);
+      pending &= ~(1u << t);
+      off = (b + t) * R::size;
       const unsigned code = code_load(bG + off);
       double f[SPL];
       row_load(bJ + off, f);
@@ -1071,7 +1316,7 @@ __global__ void __launch_bounds__(kBottomWarps * 32) k_bottom(TreeArgs a, int fi
       bool own[SPL] = {};
       if (special) {
         const int4 w = vt[t];
-        const int se = vs[t], dep = w.w & INT_MAX;
+        const int se = vs[t], dep = w.w & kDepthBits;
 #pragma unroll
         for (int k = 0; k < SPL; k++) {
           if (b + t == srow[k]) f[k] = lds64(bJ + off + 8 * k);  // the source itself is no target
@@ -1156,7 +1401,7 @@ __global__ void __launch_bounds__(kBottomWarps * 32) k_bottom(TreeArgs a, int fi
     for (int t0 = 0; t0 < m; t0 += 8) {
       const int t = t0 + (lane >> 2);
       const uint32_t ro = base + (b + min(t, m - 1)) * R::size;
-      const unsigned leads = t < m ? (unsigned)lds32(ro + R::lead) : 0;
+      const unsigned leads = t < m && (up >> t & 1) ? (unsigned)lds32(ro + R::lead) : 0;
       double z[SPL] = {};
       if (leads) {
 #pragma unroll
@@ -1186,6 +1431,9 @@ __global__ void __launch_bounds__(kBottomWarps * 32) k_bottom(TreeArgs a, int fi
     }
     __syncwarp();
   }
+  const int ne = a.xoff[r + m] - ebase;
+  for (int i = lane; i < ne; i += 32)
+    if (leaf_units[warp][i]) atomicAdd(a.Bd + ebase + i, (double)leaf_units[warp][i] * kGroup);
 }
 
 // ------------------------------------------------------------------------------- unpack, finish
@@ -1409,15 +1657,13 @@ inline unsigned blocks_for(int64_t threads, int per) { return (unsigned)std::max
 struct TreePlan {
   TreeArgs args{};  // without the per-launch fields
   int nbot = 0, up_warps = 0;
-  std::vector<int32_t> level_first;  // first piece of each trunk level, end
-  std::vector<int32_t> level_len;    // longest piece of each trunk level
+  std::vector<int32_t> level_class;  // 4 per trunk level: first piece, of at most 16, of at most 8 vertices, end
   struct BotClass {
     int first, end, rows;
   };
   std::vector<BotClass> bot_class;
   std::vector<int64_t> tri_first;    // first triangle of each unpack level, end
   int4 *tri = nullptr;
-  unsigned absent = 0;               // key of a missing entry: above every distance
   int64_t *tri_at = nullptr;         // tri_first on the device
   int32_t *owner = nullptr;          // per edge its lower end
   int tail_level = 0;                // levels from here on hold at most kTailLevel triangles each
@@ -1503,8 +1749,11 @@ static TreeShape tree_shape(const Index &ix, const std::vector<int64_t> &soff) {
   s.level_first.assign((size_t)levels + 1, 0);
   for (const P &p : ps) s.level_first[p.level + 1]++;
   for (int32_t l = 0; l < levels; l++) s.level_first[l + 1] += s.level_first[l];
-  std::vector<int32_t> at(s.level_first.begin(), s.level_first.end()), by_level(ps.size());
-  for (size_t i = 0; i < ps.size(); i++) by_level[at[ps[i].level]++] = (int32_t)i;
+  std::vector<int32_t> by_level(ps.size());  // by level, longest first
+  for (size_t i = 0; i < ps.size(); i++) by_level[i] = (int32_t)i;
+  std::stable_sort(by_level.begin(), by_level.end(), [&](int32_t x, int32_t y) {
+    return ps[x].level != ps[y].level ? ps[x].level < ps[y].level : ps[x].v.size() > ps[y].v.size();
+  });
   for (int32_t id : by_level) {
     const int32_t first = (int32_t)s.trunk_tid.size(), np = (int32_t)s.piece.size();
     for (int32_t t : ps[id].v) {
@@ -1559,11 +1808,14 @@ void tree_build(Handle &h, DeviceState *d, const std::vector<int64_t> &soff, con
     const int32_t n = ix.n;
     const TreeShape s = tree_shape(ix, soff);
     p->nbot = (int)s.bot.size();
-    p->level_first = s.level_first;
-    for (size_t l = 0; l + 1 < s.level_first.size(); l++) {
-      int32_t len = 0;
-      for (int32_t q = s.level_first[l]; q < s.level_first[l + 1]; q++) len = std::max(len, s.piece[q].y - s.piece[q].x);
-      p->level_len.push_back(len);
+    for (size_t l = 0; l + 1 < s.level_first.size(); l++) {  // (longest first, see tree_shape)
+      int32_t q = s.level_first[l];
+      p->level_class.push_back(q);
+      for (int32_t lim : {16, 8}) {
+        while (q < s.level_first[l + 1] && s.piece[q].y - s.piece[q].x > lim) q++;
+        p->level_class.push_back(q);
+      }
+      p->level_class.push_back(s.level_first[l + 1]);
     }
     for (int i = 0; i < p->nbot;) {  // bottoms come largest first: launches of 32, 24, 16 and 8 rows
       const int rows = (s.bot[i].y + s.bot[i].z + 7) & ~7;
@@ -1577,7 +1829,7 @@ void tree_build(Handle &h, DeviceState *d, const std::vector<int64_t> &soff, con
     a.NT = (int)s.trunk_tid.size();
     a.bits = bits;
     a.dist_lim = (unsigned)(dmax + 1);
-    p->absent = ((unsigned)(lim - 2 - dmax) << bits) | ((1u << bits) - 2u);
+    a.absent = ((unsigned)(lim - 2 - dmax) << bits) | ((1u << bits) - 2u);
     std::vector<int32_t> xoff(soff.begin(), soff.end());
     std::vector<int4> tmeta((size_t)a.NT);
     std::vector<int2> tsub((size_t)a.NT);
@@ -1734,6 +1986,8 @@ void tree_build(Handle &h, DeviceState *d, const std::vector<int64_t> &soff, con
 // device bytes of one group of sources
 static size_t group_bytes(const TreeArgs &a) { return ((size_t)a.NT * (4 + 4 + 4 + 8) + (size_t)a.H * (4 + 4 + 8)) * kGroup; }
 
+constexpr int64_t kWideCtas = 148 * 12;  // (piece, group) pairs from which a level is wide
+
 // Groups of sources that the per-source scratch holds, at most kMaxGroups.
 constexpr int kMaxGroups = 128;
 static int groups_fit(const DeviceState *d) {
@@ -1772,28 +2026,15 @@ bool tree_disable(DeviceState *d) {
   return true;
 }
 
-template <int GB>
-static void launch_down(const TreeArgs &a, int piece0, int pieces, int pl, int threads, cudaStream_t st) {
-  const size_t smem = (size_t)GB * pl * kGroup * 12;
-  CK(cudaFuncSetAttribute(k_trunk_down<GB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  k_trunk_down<GB><<<dim3(pieces, (a.ng + GB - 1) / GB), threads, smem, st>>>(a, piece0, pl);
-}
-template <int GB>
-static void launch_up(const TreeArgs &a, int piece0, int pieces, int pl, int threads, cudaStream_t st) {
-  const size_t smem = (size_t)GB * pl * kGroup * 12;
-  CK(cudaFuncSetAttribute(k_trunk_up<GB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  k_trunk_up<GB><<<dim3(pieces, (a.ng + GB - 1) / GB), threads, smem, st>>>(a, piece0, pl);
-}
-
 // The bottoms [first, end) of at most `rows` rows: the warps of a CTA share a bottom's edges, and a
 // CTA takes more groups one after another while there are CTAs enough.
-static void launch_bottom(const TreeArgs &a, int first, int end, int rows, unsigned absent, cudaStream_t st) {
+static void launch_bottom(const TreeArgs &a, int first, int end, int rows, cudaStream_t st) {
   const int warps = std::min(kBottomWarps, a.ng);
   int gpc = warps;
   while (gpc < 64 && (int64_t)(end - first) * ((a.ng + 2 * gpc - 1) / (2 * gpc)) >= 148 * 24) gpc *= 2;
   const size_t smem = (size_t)warps * rows * RowLayout::size;
   CK(cudaFuncSetAttribute(k_bottom, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  k_bottom<<<dim3(end - first, (a.ng + gpc - 1) / gpc), warps * 32, smem, st>>>(a, first, rows, gpc, absent);
+  k_bottom<<<dim3(end - first, (a.ng + gpc - 1) / gpc), warps * 32, smem, st>>>(a, first, rows, gpc);
 }
 
 void launch_tree(const Handle &h, DeviceState *d, const int32_t *d_src_tid, int32_t ns, cudaStream_t st) {
@@ -1804,7 +2045,7 @@ void launch_tree(const Handle &h, DeviceState *d, const int32_t *d_src_tid, int3
     d->launches++;
   };
   const int fit = groups_fit(d);
-  const int levels = (int)p.level_len.size();
+  const int levels = (int)p.level_class.size() / 4;
   std::pair<cudaEvent_t, cudaEvent_t> ev{};
   for (int32_t off = 0; off < ns; off += fit * kGroup) {
     TreeArgs a = p.args;
@@ -1839,20 +2080,33 @@ void launch_tree(const Handle &h, DeviceState *d, const int32_t *d_src_tid, int3
       k_up_rows<<<(a.ng * kGroup + p.up_warps - 1) / p.up_warps, p.up_warps * 32, smem, st>>>(a);
       launched();
     }
-    // a CTA takes one piece, for two groups when there are CTAs enough
-    auto pair_of = [&](int pieces) { return a.ng > 1 && (int64_t)pieces * a.ng >= 148 * 8; };
     for (int l = 0; l < levels; l++) {
-      const int pieces = p.level_first[l + 1] - p.level_first[l], pl = p.level_len[l];
-      launch_down<1>(a, p.level_first[l], pieces, pl, pair_of(pieces) ? 256 : 512, st);
-      launched();
+      const int32_t *c = p.level_class.data() + 4 * l;
+      if ((int64_t)(c[3] - c[0]) * a.ng < kWideCtas) {
+        k_trunk_down_narrow<<<dim3(c[3] - c[0], a.ng), kPieceLen * 32, 0, st>>>(a, c[0]);
+        launched();
+        continue;
+      }
+      if (c[1] > c[0]) {
+        k_trunk_down<32><<<dim3(c[1] - c[0], a.ng), Wide<32>::warps * 32, 0, st>>>(a, c[0]);
+        launched();
+      }
+      if (c[2] > c[1]) {
+        k_trunk_down<16><<<dim3(c[2] - c[1], a.ng), Wide<16>::warps * 32, 0, st>>>(a, c[1]);
+        launched();
+      }
+      if (c[3] > c[2]) {
+        k_trunk_down<8><<<dim3(c[3] - c[2], a.ng), Wide<8>::warps * 32, 0, st>>>(a, c[2]);
+        launched();
+      }
     }
     if (a.ng > 4) {
       for (const TreePlan::BotClass &c : p.bot_class) {
-        launch_bottom(a, c.first, c.end, c.rows, p.absent, st);
+        launch_bottom(a, c.first, c.end, c.rows, st);
         launched();
       }
     } else if (p.nbot) {
-      launch_bottom(a, 0, p.nbot, p.bot_class[0].rows, p.absent, st);
+      launch_bottom(a, 0, p.nbot, p.bot_class[0].rows, st);
       launched();
     }
     if (d->profiling) {
@@ -1861,9 +2115,24 @@ void launch_tree(const Handle &h, DeviceState *d, const int32_t *d_src_tid, int3
       CK(cudaEventRecord(ev.first, st));
     }
     for (int l = levels - 1; l >= 0; l--) {
-      const int pieces = p.level_first[l + 1] - p.level_first[l], pl = p.level_len[l];
-      launch_up<1>(a, p.level_first[l], pieces, pl, pair_of(pieces) ? 256 : 512, st);
-      launched();
+      const int32_t *c = p.level_class.data() + 4 * l;
+      if ((int64_t)(c[3] - c[0]) * a.ng < kWideCtas) {
+        k_trunk_up_narrow<<<dim3(c[3] - c[0], a.ng), kPieceLen * 32, 0, st>>>(a, c[0]);
+        launched();
+        continue;
+      }
+      if (c[1] > c[0]) {
+        k_trunk_up<32><<<dim3(c[1] - c[0], a.ng), Wide<32>::warps * 32, 0, st>>>(a, c[0]);
+        launched();
+      }
+      if (c[2] > c[1]) {
+        k_trunk_up<16><<<dim3(c[2] - c[1], a.ng), Wide<16>::warps * 32, 0, st>>>(a, c[1]);
+        launched();
+      }
+      if (c[3] > c[2]) {
+        k_trunk_up<8><<<dim3(c[3] - c[2], a.ng), Wide<8>::warps * 32, 0, st>>>(a, c[2]);
+        launched();
+      }
     }
     {
       const size_t smem = (size_t)a.H * 20;
