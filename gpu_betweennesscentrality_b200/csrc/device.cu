@@ -2319,8 +2319,10 @@ static void launch_label(const Handle &h, DeviceState *d, int buf, const int32_t
   a.guard = guard;
   const int groups = (ns + p.G - 1) / p.G;
   CK(cudaMemsetAsync(d->maxhop[buf], 0, (size_t)ns * 4, st));
-  k_src_rows<<<(ns + 127) / 128, 128, 0, st>>>(src, ns, d->depth, d->parent, d->send, d->hmax_pad, d->src_rows[buf]);
-  CK(cudaGetLastError());
+  if (!tree_source_rows(d, src, ns, d->hmax_pad, d->src_rows[buf], st)) {
+    k_src_rows<<<(ns + 127) / 128, 128, 0, st>>>(src, ns, d->depth, d->parent, d->send, d->hmax_pad, d->src_rows[buf]);
+    CK(cudaGetLastError());
+  }
   d->launches++;
   std::pair<cudaEvent_t, cudaEvent_t> ev{};
   if (d->profiling) {
@@ -3747,8 +3749,10 @@ void host_bc_source_static(Handle &h, int32_t source0, double *d_bc_vid, void *s
     const LabelPlan p = plan_label(h, d, 1, true);
     LabelArgs la{};
     int32_t *src_rows = reinterpret_cast<int32_t *>(base + kStaticSrcRows);
-    k_src_rows<<<1, 32, 0, st>>>(src, 1, d->depth, d->parent, d->send, d->hmax_pad, src_rows);
-    CK(cudaGetLastError());
+    if (!tree_source_rows(d, src, 1, d->hmax_pad, src_rows, st)) {
+      k_src_rows<<<1, 32, 0, st>>>(src, 1, d->depth, d->parent, d->send, d->hmax_pad, src_rows);
+      CK(cudaGetLastError());
+    }
     la.dis = d->dis;
     la.ch = d->ch;
     la.src_rows = src_rows;

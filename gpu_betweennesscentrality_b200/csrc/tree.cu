@@ -51,8 +51,10 @@ constexpr unsigned kAll = 0xffffffffu;
 constexpr unsigned kNoKey = 0xffffffffu;
 constexpr int kGroup = 64;           // sources a warp takes: two neighbouring ones per lane
 constexpr int kPieceLen = 32;        // trunk vertices per piece
-constexpr int kBottomRows = 24;      // shared-memory rows of a bottom subtree (its separator + its vertices)
-constexpr int kBottomEdges = 128;    // ... and its edges (grids of 2k to 1M vertices: at most 74)
+// a bottom subtree: rows in shared memory (its separator and its vertices with descendants), vertices, edges
+constexpr int kBottomRows = 16;
+constexpr int kBottomVerts = 64;
+constexpr int kBottomEdges = 224;
 constexpr int kMaxUnpackLevels = 1024;
 
 struct TreeArgs {
@@ -68,8 +70,11 @@ struct TreeArgs {
   const int2 *tsub;                // per trunk vertex (subtree end, depth - 1)
   const int4 *piece;               // (first trunk index, end, trunk index of the parent or -1, 0)
   const int32_t *piece_of;         // per trunk vertex
+  const int32_t *chain_off;        // per piece: the pieces above it, root first, and itself, as
+  const int2 *chain;               // (first trunk index, depth - 1 of that vertex)
   const int32_t *tidx_of;          // per tid: trunk index, or -1 - bottom
-  const int4 *bot;                 // bottoms: (root tid, size, separator size, 0)
+  const int4 *bot;                 // bottoms: (root tid, size, separator size, rows)
+  const uint8_t *row_of;           // per tid in a bottom: its row, 0xff without descendants
   const int32_t *depth, *parent, *send;
   const int64_t *lab_off;          // label rows (MHL): distances, shifted by lab_bits, and (count, hop)
   const int32_t *lab_dis;
@@ -240,21 +245,53 @@ __global__ void k_up_rows(TreeArgs a) {
   }
 }
 
+// The label kernels' source rows (k_src_rows: a source's ancestors, root first, then their subtree
+// ends) from the plan: a warp per source, a run of ancestors per step instead of one parent link
+// after another (a chain of 477 dependent loads at 50k vertices).
+__global__ void k_source_rows(TreeArgs a, int stride, int32_t *rows) {
+  const int slot = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (slot >= a.ns) return;
+  int32_t *lo = rows + (size_t)slot * 2 * stride, *hi = lo + stride;
+  int y = a.src[slot], j = a.depth[y] - 1, i = a.tidx_of[y];
+  while (i < 0 && j >= 0) {
+    if (lane == 0) {
+      lo[j] = y;
+      hi[j] = a.send[y];
+    }
+    j--;
+    y = a.parent[y];
+    i = y >= 0 ? a.tidx_of[y] : 0;
+  }
+  if (j < 0) return;
+  const int pc = a.piece_of[i], c0 = a.chain_off[pc], c1 = a.chain_off[pc + 1];
+#pragma unroll 4
+  for (int c = c0; c < c1; c++) {
+    const int2 run = a.chain[c];
+    const int end = c + 1 < c1 ? a.chain[c + 1].y : j + 1;
+    if (run.y + lane < end) {
+      lo[run.y + lane] = a.tmeta[run.x + lane].w;
+      hi[run.y + lane] = a.tsub[run.x + lane].x;
+    }
+  }
+}
+
 // Reverse of the U rows, a CTA per source, root first: the flow of y is its seed plus its share of the
 // flow of the separator entries x with U(y) + L = U(x).  Each warp takes a block of 32 ancestors and
 // collects the entries that hold (independent loads, the next ancestor's in flight); one warp then
 // applies the blocks in order in shared memory, and all add the shortcuts' flow.
-constexpr int kBackWarps = 8;
-constexpr int kBackHits = 192;  // entries collected per block; a block with more is done by one warp in turns
+// Many sources: four warps, so that more CTAs wait at a time; few: eight, for the shorter wait.
+constexpr int kBackHits = 160;  // entries collected per block; a block with more is done by one warp in turns
+template <int BW>
 struct BackShared {
-  int2 hit[kBackWarps][kBackHits];  // (edge, x's depth | y's depth << 16)
-  double ratio[kBackWarps][kBackHits];
-  int count[kBackWarps];
+  int2 hit[BW][kBackHits];  // (edge, x's depth | y's depth << 16)
+  double ratio[BW][kBackHits];
+  int count[BW];
 };
 
-__global__ void __launch_bounds__(kBackWarps * 32) k_up_back(TreeArgs a) {
+template <int BW>
+__global__ void __launch_bounds__(BW * 32) k_up_back(TreeArgs a) {
   extern __shared__ double sm_back[];
-  __shared__ BackShared sh;
+  __shared__ BackShared<BW> sh;
   if (__syncthreads_or(wrapped(a))) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nt = blockDim.x;
   const int slot = blockIdx.x;
@@ -268,20 +305,21 @@ __global__ void __launch_bounds__(kBackWarps * 32) k_up_back(TreeArgs a) {
     uc[q] = a.Uc[gbase + (size_t)q * kGroup];
     ub[q] = a.seed[gbase + (size_t)q * kGroup];
   }
-  if (warp == 0) {
+  {
     int j = h - 1, y = s, i = a.tidx_of[y];
     while (i < 0 && j >= 0) {
-      if (lane == 0) path[j] = -1 - y;
+      if (threadIdx.x == 0) path[j] = -1 - y;
       j--;
       y = a.parent[y];
       i = y >= 0 ? a.tidx_of[y] : 0;
     }
-    while (j >= 0) {
-      const int4 pc = a.piece[a.piece_of[i]];
-      const int cnt = i - pc.x + 1;
-      if (lane < cnt) path[j - (cnt - 1) + lane] = pc.x + lane;
-      j -= cnt;
-      i = pc.z;
+    if (j >= 0) {  // ancestors in the trunk: a run of trunk indices per piece
+      const int pc = a.piece_of[i], c0 = a.chain_off[pc], c1 = a.chain_off[pc + 1];
+      for (int c = c0 + warp; c < c1; c += BW) {
+        const int2 run = a.chain[c];
+        const int end = c + 1 < c1 ? a.chain[c + 1].y : j + 1;
+        if (run.y + lane < end) path[run.y + lane] = run.x + lane;
+      }
     }
   }
   __syncthreads();
@@ -367,7 +405,7 @@ __global__ void __launch_bounds__(kBackWarps * 32) k_up_back(TreeArgs a) {
       if (f != 0.0) atomicAdd(((int)((unsigned)t.y >> 16) == h - 1 ? a.Bs : a.Bu) + t.x, f);
     }
   };
-  for (int r0 = 0; r0 < h; r0 += kBackWarps * 32) {
+  for (int r0 = 0; r0 < h; r0 += BW * 32) {
     const int q0 = r0 + warp * 32;
     int done = 32;
     if (q0 < h) done = collect(warp, q0, 0);
@@ -375,11 +413,11 @@ __global__ void __launch_bounds__(kBackWarps * 32) k_up_back(TreeArgs a) {
     const bool crowded = __syncthreads_or(done < 32);
     if (!crowded) {
       if (warp == 0)
-        for (int w = 0; w < kBackWarps; w++) apply(w);
+        for (int w = 0; w < BW; w++) apply(w);
       __syncthreads();
       add(warp, lane, 32);
     } else if (warp == 0) {  // more entries than the lists hold: one warp, list by list
-      for (int w = 0; w < kBackWarps; w++)
+      for (int w = 0; w < BW; w++)
         for (int from = 0; r0 + w * 32 < h && from < 32;) {
           __syncwarp();
           int next = collect(0, r0 + w * 32, from);
@@ -996,21 +1034,22 @@ __global__ void __launch_bounds__(kPieceLen * 32) k_trunk_up_narrow(TreeArgs a, 
 }
 
 // ------------------------------------------------------------------------------- bottoms
-// A whole subtree below the trunk for a group at a time in a warp's shared memory: rows
-// 0..b-1 are the root's separator (trunk vertices), then the subtree in preorder.  Down then up, so
-// nothing of the subtree is written to global memory.  Distances are kept shifted (a key without its
-// index), and an entry's index in the keys is its row + 1 (0: U), so the row a lane's paths come from
-// needs no lookup.  On the way up most vertices hand everything to one entry in all lanes (at 50k 1.1
-// to 1.3 different entries per vertex and warp): that entry's flow stays in the finished row and is
-// summed after the pass, eight rows at a time, instead of by a warp-wide sum per vertex.
+// A whole subtree below the trunk for a group at a time in a warp's shared memory: rows 0..b-1 are
+// the root's separator (trunk vertices), then the subtree's vertices with descendants in preorder.
+// Down then up, so nothing of the subtree is written to global memory.  Distances are kept shifted (a
+// key without its index), and an entry's index in the keys is its row + 1 (0: U), so the row a lane's
+// paths come from needs no lookup.  A vertex without descendants (44 % of them) has no row: nobody
+// reads it and its flow is 1 per source, so it is done on the way down, and where all lanes hand
+// everything to one entry, as most do, only that entry's row and a counter change.  On the way up
+// most vertices, too, hand everything to one entry in all lanes (at 50k 1.1 to 1.3 different entries
+// per vertex and warp): that entry's flow stays in the finished row and is summed after the pass,
+// eight rows at a time, instead of by a warp-wide sum per vertex.
 //
-// A vertex without descendants (44 % of them) that hands everything to one entry in all lanes is done
-// at once on the way down: its flow is 1 per source, and nobody reads its row.
-//
-// The pass is bound by instruction issue, so shared memory is addressed by 32-bit offsets (ld.shared
-// / st.shared); a row's block holds delta (f64), distance, count and argument of the warp's sources.
+// The pass is bound by instruction issue and by the warps that shared memory leaves room for, so
+// shared memory is addressed by 32-bit offsets (ld.shared / st.shared); a row's block holds delta
+// (f64), distance, count and argument of the warp's sources.
 constexpr int kTieCode = 0xff, kSkipCode = 0xfe;  // arguments that are no row: a tie, a lane without a source
-constexpr int kBottomPairs = (kBottomEdges + kBottomRows) / 2 + 1;
+constexpr int kBottomPairs = (kBottomEdges + kBottomVerts) / 2 + 1;
 constexpr int kBottomWarps = 2;
 constexpr int kLeadFull = 1 << 16;  // deferred sum: every lane, the rows' delta + 1 each
 constexpr int kManyCounts = INT_MIN, kLeaf = 1 << 30, kDepthBits = kLeaf - 1;  // in a vertex's fourth word
@@ -1064,33 +1103,47 @@ __device__ __forceinline__ void code_store(uint32_t p, unsigned v) {
 __global__ void __launch_bounds__(kBottomWarps * 32) k_bottom(TreeArgs a, int first, int rows, int gpc) {
   extern __shared__ int4 sm_b[];
   using R = RowLayout;
-  constexpr int SPL = 2;
-  __shared__ int4 ep[kBottomPairs];           // two edges: (x row offset, key) twice
-  __shared__ int2 er[kBottomEdges];           // an edge: (x row + 1, count)
-  __shared__ int4 vt[kBottomRows + 1];        // a vertex: (address of its first pair, end, first edge | edges << 16, depth - 1 | kLeaf | kManyCounts)
+  __shared__ int4 ep[kBottomPairs];      // two edges: (x row offset, key) twice
+  __shared__ int4 vt[kBottomVerts + 1];  // a vertex: (address of its first pair, end, first edge | edges << 16, depth - 1 | kLeaf | kManyCounts)
+  __shared__ int vs[kBottomVerts], sep[kBottomRows];  // subtree end, trunk index
+  __shared__ uint8_t emap[kBottomVerts][kBottomRows];  // edge of (vertex, x row)
+  __shared__ uint8_t vertex_of[kBottomRows];           // of a row (less b)
   __shared__ uint8_t leaf_units[kBottomWarps][kBottomEdges];  // groups (at most 64) whose leaf handed everything to the edge
-  __shared__ int vs[kBottomRows], sep[kBottomRows];  // subtree end, trunk index
-  __shared__ uint8_t emap[kBottomRows][kBottomRows + 4];  // edge of (vertex, x row)
   if (__syncthreads_or(wrapped(a))) return;
   const int4 bt = a.bot[first + blockIdx.x];
-  const int r = bt.x, m = bt.y, b = bt.z;
+  const int r = bt.x, m = bt.y, b = bt.z, nr = bt.w - bt.z;  // nr: vertices with descendants
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   const int ebase = a.xoff[r];
   const uint32_t ep0 = (uint32_t)__cvta_generic_to_shared(ep), vt0 = (uint32_t)__cvta_generic_to_shared(vt);
-  if (warp == 0) {
-    const int e0 = lane < m ? a.xoff[r + lane] - ebase : 0, k = lane < m ? a.xoff[r + lane + 1] - ebase - e0 : 0;
-    const int pairs = lane < m ? max(1, (k + 1) >> 1) : 0;  // (the tree's root has no entries: one absent pair)
-    int x = pairs;
+  if (warp == 0) {  // two vertices per lane
+    int e0[2], k[2], pairs[2];
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      const int t = 2 * lane + q;
+      e0[q] = t < m ? a.xoff[r + t] - ebase : 0;
+      k[q] = t < m ? a.xoff[r + t + 1] - ebase - e0[q] : 0;
+      pairs[q] = t < m ? max(1, (k[q] + 1) >> 1) : 0;  // (the tree's root has no entries: one absent pair)
+    }
+    int x = pairs[0] + pairs[1];
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int z = __shfl_up_sync(kAll, x, o);
       if (lane >= o) x += z;
     }
-    if (lane < m)
-      vt[lane] = make_int4((int)ep0 + 16 * (x - pairs), (int)ep0 + 16 * x, e0 | (k << 16), a.depth[r + lane] - 1);
+    int pos = (int)ep0 + 16 * (x - pairs[0] - pairs[1]);
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      const int t = 2 * lane + q;
+      if (t < m) {
+        vt[t] = make_int4(pos, pos + 16 * pairs[q], e0[q] | (k[q] << 16), a.depth[r + t] - 1);
+        vs[t] = a.send[r + t];
+        const int row = a.row_of[r + t];
+        if (row != 0xff) vertex_of[row - b] = (uint8_t)t;
+      }
+      pos += 16 * pairs[q];
+    }
     if (lane == 0) vt[m] = make_int4((int)ep0, (int)ep0, 0, 0);  // read ahead, not used
   }
-  for (int i = threadIdx.x; i < m; i += blockDim.x) vs[i] = a.send[r + i];
   for (int i = threadIdx.x; i < b; i += blockDim.x) sep[i] = a.etr[ebase + i];
   for (int i = threadIdx.x; i < kBottomWarps * kBottomEdges; i += blockDim.x) (&leaf_units[0][0])[i] = 0;
   __syncthreads();
@@ -1102,9 +1155,7 @@ __global__ void __launch_bounds__(kBottomWarps * 32) k_bottom(TreeArgs a, int fi
       const int2 x = lane < k ? a.ex[ebase + e0 + lane] : make_int2(0, (int)a.absent);
       reinterpret_cast<int2 *>(ep + (((uint32_t)v.x - ep0) >> 4))[lane] = make_int2(x.x * R::size, x.y);
       if (lane < k) {
-        const int c = a.eC[ebase + e0 + lane];
-        many = c > 1;
-        er[e0 + lane] = make_int2(x.x + 1, c);
+        many = a.eC[ebase + e0 + lane] > 1;
         emap[t][x.x] = (uint8_t)(e0 + lane);
       }
     }
@@ -1113,12 +1164,12 @@ __global__ void __launch_bounds__(kBottomWarps * 32) k_bottom(TreeArgs a, int fi
   }
   __syncthreads();
   const uint32_t base = (uint32_t)__cvta_generic_to_shared(sm_b) + (uint32_t)warp * (uint32_t)rows * R::size;
-  const uint32_t bJ = base + lane * 8 * SPL, bD = base + R::D + lane * 4 * SPL, bG = base + R::G + lane * SPL;
+  const uint32_t bJ = base + lane * 16, bD = base + R::D + lane * 8, bS = base + R::S + lane * 8, bG = base + R::G + lane * 2;
   const unsigned mask = (1u << a.bits) - 1u;
   const int gend = min(a.ng, ((int)blockIdx.y + 1) * gpc);
   // the next group's sources and first separator rows
-  int ns[SPL], nsi[SPL];
-  bool nlive[SPL];
+  int ns[2], nsi[2];
+  bool nlive[2];
   uint2 nd[kAhead], nc[kAhead];
   auto load_ahead = [&](int g) {
     lane_sources(a, g, lane, ns, nlive);
@@ -1130,40 +1181,41 @@ __global__ void __launch_bounds__(kBottomWarps * 32) k_bottom(TreeArgs a, int fi
         nc[q] = __ldg(reinterpret_cast<const uint2 *>(a.S + gt + (size_t)sep[q] * kGroup));
       }
 #pragma unroll
-    for (int k = 0; k < SPL; k++) nsi[k] = a.tidx_of[ns[k]];
+    for (int k = 0; k < 2; k++) nsi[k] = a.tidx_of[ns[k]];
   };
   const int gfirst = blockIdx.y * gpc + warp;
   if (gfirst < gend) load_ahead(gfirst);
   for (int g = gfirst; g < gend; g += nw) {
-    int s[SPL], srow[SPL], si[SPL];
-    bool live[SPL];
+    int s[2], srow[2], si[2];
+    bool live[2];
     const size_t gt = (size_t)g * a.NT * kGroup + 2 * lane, gu = (size_t)g * a.H * kGroup + 2 * lane;
     bool in_any = false, odd = false;
 #pragma unroll
-    for (int k = 0; k < SPL; k++) {
+    for (int k = 0; k < 2; k++) {
       s[k] = ns[k];
       si[k] = nsi[k];
       live[k] = nlive[k];
-      srow[k] = r <= s[k] && s[k] < r + m ? b + s[k] - r : -1;  // the row of this lane's own source
-      in_any |= srow[k] >= 0;
+      const bool in = r <= s[k] && s[k] < r + m;
+      srow[k] = in ? a.row_of[s[k]] : 0xff;  // the row of this lane's own source, if it has one
+      in_any |= in;
     }
-    const double zero[SPL] = {};
-    const uint32_t none[SPL] = {};
+    const double zero[2] = {};
+    const uint32_t none[2] = {};
     if (b == 0) row_store(bD, none);  // the whole tree: an absent entry of its root reads this row
 #pragma unroll
     for (int q = 0; q < kAhead; q++)
       if (q < b) {
-        const uint32_t d[SPL] = {nd[q].x, nd[q].y}, c[SPL] = {nc[q].x, nc[q].y};
+        const uint32_t d[2] = {nd[q].x, nd[q].y}, c[2] = {nc[q].x, nc[q].y};
         row_store(bD + q * R::size, d);
-        row_store(bD + (R::S - R::D) + q * R::size, c);
+        row_store(bS + q * R::size, c);
         row_store(bJ + q * R::size, zero);
         const int sp = sep[q];
 #pragma unroll
-        for (int k = 0; k < SPL; k++)
+        for (int k = 0; k < 2; k++)
           if (sp == si[k]) srow[k] = q;
       }
     for (int i = kAhead; i < b; i += 4) {  // the separator's other rows, four loads of each in flight
-      uint32_t d[4][SPL], c[4][SPL];
+      uint32_t d[4][2], c[4][2];
       int sp[4];
 #pragma unroll
       for (int q = 0; q < 4; q++) {
@@ -1179,93 +1231,132 @@ __global__ void __launch_bounds__(kBottomWarps * 32) k_bottom(TreeArgs a, int fi
       for (int q = 0; q < 4; q++)
         if (i + q < b) {
           row_store(bD + (i + q) * R::size, d[q]);
-          row_store(bD + (R::S - R::D) + (i + q) * R::size, c[q]);
+          row_store(bS + (i + q) * R::size, c[q]);
           row_store(bJ + (i + q) * R::size, zero);
 #pragma unroll
-          for (int k = 0; k < SPL; k++)
+          for (int k = 0; k < 2; k++)
             if (sp[q] == si[k]) srow[k] = i + q;
         }
     }
 #pragma unroll
-    for (int k = 0; k < SPL; k++) odd |= srow[k] >= 0 || !live[k];
-    // special: some lane's source lies among these rows, or lanes without a source
-    const bool inside = __any_sync(kAll, in_any), special = __any_sync(kAll, odd);
-    unsigned over = 0, pending = m == 32 ? kAll : (1u << m) - 1u;  // vertices of the way up
-    uint32_t off = b * R::size;  // of the current row
-    int4 v = lds128(vt0), e = lds128(v.x);
-    for (int t = 0; t < m; t++, off += R::size) {
-      const int4 vn = lds128(vt0 + 16 * (t + 1));
-      unsigned m1[SPL], m2[SPL];
+    for (int k = 0; k < 2; k++) odd |= srow[k] != 0xff || !live[k];
+    // special: some lane's source lies in this subtree or among its separator, or lanes without a source
+    const bool inside = __any_sync(kAll, in_any), special = __any_sync(kAll, odd || in_any);
+    unsigned over = 0;
+
+    // What vertex t does with its flows f, distances dt, counts c and arguments x1 (0 afterwards for
+    // lanes that are done; else their entry, whose flow through the edge is still to be added).
+    auto hand_on = [&](int t, double (&f)[2], unsigned (&x1)[2], const uint32_t (&dt)[2], const uint32_t (&c)[2]) {
+      const int4 v = vt[t];
 #pragma unroll
-      for (int k = 0; k < SPL; k++) m1[k] = m2[k] = kNoKey;
+      for (int k = 0; k < 2; k++) {
+        if (special && live[k] && r + t <= s[k] && s[k] < vs[t]) {
+          const size_t u = gu + (size_t)(v.w & kDepthBits) * kGroup + k;
+          double sd = x1[k] == 0 ? f[k] : 0.0;
+          if (x1[k] == kTieCode && (unsigned)a.Ud[u] == dt[k] >> a.bits) sd = f[k] * share(1, a.Uc[u], c[k]);
+          a.seed[u] = sd;
+        }
+        if (x1[k] - 1 < (unsigned)kBottomRows) {
+          const uint32_t xo = bJ + (x1[k] - 1) * R::size + 8 * k;
+          sts64(xo, lds64(xo) + f[k]);
+          if (special && (int)x1[k] - 1 == srow[k]) {  // flow into the lane's own source counts apart
+            atomicAdd(a.Bs + ebase + emap[t][x1[k] - 1], f[k]);
+            x1[k] = 0;
+          }
+        } else if (x1[k] == kTieCode) {
+          for (int q = 0; q < v.z >> 16; q++) {
+            const int eq = (v.z & 0xffff) + q;
+            const unsigned key = (unsigned)lds32(v.x + 8 * q + 4);
+            const int xr = (int)(key & mask) - 1;
+            const uint32_t xo = (uint32_t)xr * R::size;
+            if ((uint32_t)lds32(bD + xo + 4 * k) + (key & ~mask) == dt[k]) {
+              const double fl = f[k] * share(a.eC[ebase + eq], (uint32_t)lds32(bS + xo + 4 * k), c[k]);
+              sts64(bJ + xo + 8 * k, lds64(bJ + xo + 8 * k) + fl);
+              atomicAdd((xr == srow[k] ? a.Bs : a.Bd) + ebase + eq, fl);
+            }
+          }
+          x1[k] = 0;
+        } else {
+          x1[k] = 0;
+        }
+      }
+    };
+    // the first entry that lanes still have (0: none)
+    auto leader = [&](const unsigned (&x1)[2]) -> unsigned {
+      const unsigned mine = x1[0] ? x1[0] : x1[1], any = __ballot_sync(kAll, mine != 0);
+      return any ? __shfl_sync(kAll, mine, __ffs(any) - 1) : 0u;
+    };
+
+    uint32_t off = b * R::size;  // of the next row
+    int4 v = lds128(vt0), e = lds128(v.x);
+    for (int t = 0; t < m; t++) {
+      const int4 vn = lds128(vt0 + 16 * (t + 1));
+      unsigned m1[2] = {kNoKey, kNoKey}, m2[2] = {kNoKey, kNoKey};
       if (inside) {
         const int se = vs[t];
 #pragma unroll
-        for (int k = 0; k < SPL; k++) {
+        for (int k = 0; k < 2; k++) {
           m1[k] = up_key(a, r + t <= s[k] && s[k] < se, gu + (size_t)(v.w & kDepthBits) * kGroup + k);
           m2[k] = m1[k] == kNoKey ? kNoKey : m1[k] ^ mask;
         }
       }
       uint32_t pe = v.x;
       do {
-        uint32_t d1[SPL], d2[SPL];
+        uint32_t d1[2], d2[2];
         row_load(bD + e.x, d1);
         row_load(bD + e.z, d2);
         const int4 ec = e;
         pe += 16;
         if (pe < (uint32_t)v.y) e = lds128(pe);
 #pragma unroll
-        for (int k = 0; k < SPL; k++) {
-          const unsigned v1 = d1[k] + (unsigned)ec.y, v2 = d2[k] + (unsigned)ec.w;
-          m1[k] = __vimin3_u32(m1[k], v1, v2);
-          m2[k] = __vimin3_u32(m2[k], v1 ^ mask, v2 ^ mask);
-        }
+        for (int k = 0; k < 2; k++) key_min2(m1[k], m2[k], d1[k] + (unsigned)ec.y, d2[k] + (unsigned)ec.w, mask);
       } while (pe < (uint32_t)v.y);
       e = lds128(vn.x);
-      if ((v.w & kLeaf) && !special) {
+      const bool leaf = v.w & kLeaf;
+      if (leaf && !special) {
         const unsigned x0 = m1[0] & mask;  // one entry for the lane's two sources, and for all lanes?
+        const bool one = ((m1[0] ^ m2[0]) == mask) & ((m1[1] ^ m2[1]) == mask) & ((m1[1] & mask) == x0);
         int all = 0;
-        __match_all_sync(kAll, ((m1[0] ^ m2[0]) == mask) & ((m1[1] ^ m2[1]) == mask) & ((m1[1] & mask) == x0) ? x0 : 0x100u + lane, &all);
+        __match_all_sync(kAll, one ? x0 : 0x100u + lane, &all);
         if (all) {
-          double j[SPL];
+          double j[2];
           const uint32_t xo = bJ + (x0 - 1) * R::size;
           row_load(xo, j);
-#pragma unroll
-          for (int k = 0; k < SPL; k++) j[k] += 1.0;
+          j[0] += 1.0;
+          j[1] += 1.0;
           row_store(xo, j);
           uint8_t *lu = &leaf_units[warp][emap[t][x0 - 1]];
           const uint8_t units = *lu + 1;
           __syncwarp();
           *lu = units;
-          pending &= ~(1u << t);
           v = vn;
           continue;
         }
       }
-      unsigned x1[SPL];
-      uint32_t c[SPL], dt[SPL];
+      unsigned x1[2];
+      uint32_t c[2], dt[2];
       unsigned again = 0;  // several entries reach the minimum
 #pragma unroll
-      for (int k = 0; k < SPL; k++) {
+      for (int k = 0; k < 2; k++) {
         x1[k] = m1[k] & mask;
         dt[k] = m1[k] & ~mask;
         again |= m1[k] ^ m2[k] ^ mask;
-        c[k] = (uint32_t)lds32(bD + (R::S - R::D) + 4 * k + (max(x1[k], 1u) - 1) * R::size);
+        c[k] = (uint32_t)lds32(bS + 4 * k + (max(x1[k], 1u) - 1) * R::size);
       }
       if (inside)
 #pragma unroll
-        for (int k = 0; k < SPL; k++)
+        for (int k = 0; k < 2; k++)
           if (x1[k] == 0) c[k] = a.Uc[gu + (size_t)(v.w & kDepthBits) * kGroup + k];
       if (__any_sync(kAll, (again != 0) | (v.w < 0))) {  // or counts above 1: the edges once more
 #pragma unroll
-        for (int k = 0; k < SPL; k++) {
+        for (int k = 0; k < 2; k++) {
           const bool tk = (m1[k] ^ m2[k]) != mask;
           unsigned long long cc = x1[k] == 0 ? c[k] : 0;
           for (int q = 0; q < v.z >> 16; q++) {
-            const int2 z = er[(v.z & 0xffff) + q];
-            const uint32_t xo = (uint32_t)(z.x - 1) * R::size + 4 * k, key = (uint32_t)lds32(v.x + 8 * q + 4);
-            const bool hit = tk ? (uint32_t)lds32(bD + xo) + (key & ~mask) == dt[k] : (unsigned)z.x == x1[k];
-            if (hit) cc += (unsigned long long)(unsigned)z.y * (uint32_t)lds32(bD + (R::S - R::D) + xo);
+            const unsigned key = (unsigned)lds32(v.x + 8 * q + 4);
+            const uint32_t xo = ((key & mask) - 1) * R::size + 4 * k;
+            const bool hit = tk ? (uint32_t)lds32(bD + xo) + (key & ~mask) == dt[k] : (key & mask) == x1[k];
+            if (hit) cc += (unsigned long long)(unsigned)a.eC[ebase + (v.z & 0xffff) + q] * (uint32_t)lds32(bS + xo);
             if (cc > 0x7fffffffull) {
               over = 1;
               cc = 1;
@@ -1277,117 +1368,80 @@ __global__ void __launch_bounds__(kBottomWarps * 32) k_bottom(TreeArgs a, int fi
       }
       if (special)
 #pragma unroll
-        for (int k = 0; k < SPL; k++)
+        for (int k = 0; k < 2; k++)
           if (!live[k]) x1[k] = kSkipCode;
-      row_store(bD + off, dt);
-      row_store(bD + (R::S - R::D) + off, c);
-      row_store(bJ + off, zero);
-      code_store(bG + off, x1[0] | (x1[1] << 8));
+      if (!leaf) {
+        row_store(bD + off, dt);
+        row_store(bS + off, c);
+        row_store(bJ + off, zero);
+        code_store(bG + off, x1[0] | (x1[1] << 8));
+        off += R::size;
+      } else {  // several entries, or special
+        double f[2];
+#pragma unroll
+        for (int k = 0; k < 2; k++) f[k] = r + t != s[k] ? 1.0 : 0.0;  // the source itself is no target
+        hand_on(t, f, x1, dt, c);
+        for (unsigned xl; (xl = leader(x1)) != 0;) {
+          int cnt = 0;
+#pragma unroll
+          for (int k = 0; k < 2; k++) {
+            cnt += __popc(__ballot_sync(kAll, x1[k] == xl && f[k] != 0.0));
+            if (x1[k] == xl) x1[k] = 0;
+          }
+          if (lane == 0) atomicAdd(a.Bd + ebase + emap[t][xl - 1], (double)cnt);
+        }
+      }
       v = vn;
     }
     if (over) *a.wrap = 1;
     if (g + nw < gend) load_ahead(g + nw);
-    const unsigned up = pending;
-    while (pending) {
-      const int t = 31 - __clz(pending);
-      pending &= ~(1u << t);
-      off = (b + t) * R::size;
+    for (int i = nr - 1; i >= 0; i--) {
+      off -= R::size;
       const unsigned code = code_load(bG + off);
-      double f[SPL];
+      double f[2];
       row_load(bJ + off, f);
-      const unsigned x0 = code & 0xff;
+      unsigned x1[2] = {code & 0xff, code >> 8};
       int all = 0;
       __match_all_sync(kAll, code, &all);
-#pragma unroll
-      for (int k = 0; k < SPL; k++) f[k] += 1.0;
-      if (all && !special && code == x0 * 0x101 && x0 <= kBottomRows) {  // (no U without special)
-        double j[SPL];
-        const uint32_t xo = (x0 - 1) * R::size;
+      if (all && !special && x1[0] == x1[1] && x1[0] <= kBottomRows) {  // (no U without special)
+        double j[2];
+        const uint32_t xo = (x1[0] - 1) * R::size;
         row_load(bJ + xo, j);
-#pragma unroll
-        for (int k = 0; k < SPL; k++) j[k] += f[k];
+        j[0] += f[0] + 1.0;
+        j[1] += f[1] + 1.0;
         row_store(bJ + xo, j);
-        sts32(base + off + R::lead, x0 | kLeadFull);
+        sts32(base + off + R::lead, x1[0] | kLeadFull);
         continue;
       }
-      unsigned x1[SPL];
+      const int t = vertex_of[i];
+      uint32_t dt[2], c[2];
+      row_load(bD + off, dt);
+      row_load(bS + off, c);
 #pragma unroll
-      for (int k = 0; k < SPL; k++) x1[k] = (code >> (8 * k)) & 0xff;
-      bool own[SPL] = {};
-      if (special) {
-        const int4 w = vt[t];
-        const int se = vs[t], dep = w.w & kDepthBits;
+      for (int k = 0; k < 2; k++)
+        if (r + t != s[k]) f[k] += 1.0;  // the source itself is no target
+      hand_on(t, f, x1, dt, c);
+      // two entries wait for the end, a value per lane each; any others now, one after another
+      unsigned leads = 0;
+      double w[2];
 #pragma unroll
-        for (int k = 0; k < SPL; k++) {
-          if (b + t == srow[k]) f[k] = lds64(bJ + off + 8 * k);  // the source itself is no target
-          if (live[k] && r + t <= s[k] && s[k] < se) {
-            const size_t u = gu + (size_t)dep * kGroup + k;
-            double sd = x1[k] == 0 ? f[k] : 0.0;
-            if (x1[k] == kTieCode && (unsigned)a.Ud[u] == (uint32_t)lds32(bD + off + 4 * k) >> a.bits)
-              sd = f[k] * share(1, a.Uc[u], (uint32_t)lds32(bD + (R::S - R::D) + off + 4 * k));
-            a.seed[u] = sd;
-          }
-          own[k] = x1[k] <= (unsigned)kBottomRows && x1[k] > 0 && (int)x1[k] - 1 == srow[k];  // counts apart
-        }
-      }
+      for (int j = 0; j < 2; j++) {
+        const unsigned xl = leader(x1);
+        w[j] = 0.0;
+        leads |= xl << (8 * j);
 #pragma unroll
-      for (int k = 0; k < SPL; k++)
-        if (x1[k] - 1 < (unsigned)kBottomRows) {
-          const uint32_t xo = bJ + (x1[k] - 1) * R::size + 8 * k;
-          sts64(xo, lds64(xo) + f[k]);
-          if (own[k]) {
-            atomicAdd(a.Bs + ebase + emap[t][x1[k] - 1], f[k]);
+        for (int k = 0; k < 2; k++)
+          if (xl && x1[k] == xl) {
+            w[j] += f[k];
             x1[k] = 0;
           }
-        } else if (x1[k] == kTieCode) {
-          const int4 w = vt[t];
-          const uint32_t st = (uint32_t)lds32(bD + (R::S - R::D) + off + 4 * k), dk = (uint32_t)lds32(bD + off + 4 * k);
-          for (int q = 0; q < w.z >> 16; q++) {
-            const int eq = (w.z & 0xffff) + q, xr = er[eq].x - 1;
-            const uint32_t xo = (uint32_t)xr * R::size, key = (uint32_t)lds32(w.x + 8 * q + 4);
-            if ((uint32_t)lds32(bD + xo + 4 * k) + (key & ~mask) == dk) {
-              const double fl = f[k] * share(er[eq].y, (uint32_t)lds32(bD + (R::S - R::D) + xo + 4 * k), st);
-              sts64(bJ + xo + 8 * k, lds64(bJ + xo + 8 * k) + fl);
-              atomicAdd((xr == srow[k] ? a.Bs : a.Bd) + ebase + eq, fl);
-            }
-          }
-          x1[k] = 0;
-        } else {
-          x1[k] = 0;
-        }
-      // up to SPL entries wait for the end, a value per lane each; any others now, one after another
-      unsigned leads = 0;
-      double w[SPL];
-#pragma unroll
-      for (int j = 0; j < SPL; j++) {
-        unsigned mine = 0;
-#pragma unroll
-        for (int k = 0; k < SPL; k++) mine = mine ? mine : x1[k];
-        const unsigned any = __ballot_sync(kAll, mine != 0);
-        w[j] = 0.0;
-        if (any) {
-          const unsigned xl = __shfl_sync(kAll, mine, __ffs(any) - 1);
-          leads |= xl << (8 * j);
-#pragma unroll
-          for (int k = 0; k < SPL; k++)
-            if (x1[k] == xl) {
-              w[j] += f[k];
-              x1[k] = 0;
-            }
-        }
       }
       row_store(bJ + off, w);
       sts32(base + off + R::lead, leads);
-      for (;;) {
-        unsigned mine = 0;
-#pragma unroll
-        for (int k = 0; k < SPL; k++) mine = mine ? mine : x1[k];
-        const unsigned any = __ballot_sync(kAll, mine != 0);
-        if (!any) break;
-        const unsigned xl = __shfl_sync(kAll, mine, __ffs(any) - 1);
+      for (unsigned xl; (xl = leader(x1)) != 0;) {
         double z = 0.0;
 #pragma unroll
-        for (int k = 0; k < SPL; k++)
+        for (int k = 0; k < 2; k++)
           if (x1[k] == xl) {
             z += f[k];
             x1[k] = 0;
@@ -1398,35 +1452,35 @@ __global__ void __launch_bounds__(kBottomWarps * 32) k_bottom(TreeArgs a, int fi
     }
     __syncwarp();
     // the deferred sums: eight rows at a time, four lanes of eight columns each
-    for (int t0 = 0; t0 < m; t0 += 8) {
-      const int t = t0 + (lane >> 2);
-      const uint32_t ro = base + (b + min(t, m - 1)) * R::size;
-      const unsigned leads = t < m && (up >> t & 1) ? (unsigned)lds32(ro + R::lead) : 0;
-      double z[SPL] = {};
+    for (int i0 = 0; i0 < nr; i0 += 8) {
+      const int i = min(i0 + (lane >> 2), nr - 1);
+      const uint32_t ro = base + (b + i) * R::size;
+      const unsigned leads = i0 + (lane >> 2) < nr ? (unsigned)lds32(ro + R::lead) : 0;
+      double z[2] = {};
       if (leads) {
 #pragma unroll
-        for (int c = 0; c < 8; c++) {
-          double x[SPL];
-          row_load(ro + ((lane & 3) * 8 + c) * 8 * SPL, x);
-#pragma unroll
-          for (int k = 0; k < SPL; k++) z[k] += x[k];
+        for (int q = 0; q < 8; q++) {
+          double x[2];
+          row_load(ro + ((lane & 3) * 8 + q) * 16, x);
+          z[0] += x[0];
+          z[1] += x[1];
         }
       }
       if (leads & kLeadFull) z[0] += z[1];  // one entry: both values of a lane are its
 #pragma unroll
-      for (int j = 0; j < SPL; j++) {
+      for (int j = 0; j < 2; j++) {
         z[j] += __shfl_xor_sync(kAll, z[j], 1);
         z[j] += __shfl_xor_sync(kAll, z[j], 2);
         const unsigned x = (leads >> (8 * j)) & 0xff;
         if (x && (lane & 3) == j)
-          atomicAdd(a.Bd + ebase + emap[t][x - 1], leads & kLeadFull ? z[j] + (double)kGroup : z[j]);
+          atomicAdd(a.Bd + ebase + emap[vertex_of[i]][x - 1], leads & kLeadFull ? z[j] + (double)kGroup : z[j]);
       }
     }
     for (int i = 0; i < b; i++) {
-      double z[SPL];
+      double z[2];
       row_load(bJ + i * R::size, z);
 #pragma unroll
-      for (int k = 0; k < SPL; k++)
+      for (int k = 0; k < 2; k++)
         if (z[k] != 0.0) atomicAdd(a.J + gt + (size_t)sep[i] * kGroup + k, z[k]);
     }
     __syncwarp();
@@ -1511,7 +1565,7 @@ __global__ void k_sort_edges(const int64_t *__restrict__ soff, const int4 *__res
 // per-edge references once the trunk and bottoms are known; edges that cannot carry a shortest path
 // (L above every distance) are clamped so that keys stay in 32 bits
 __global__ void k_edge_refs(const int32_t *__restrict__ xoff, const int32_t *__restrict__ xtid, const int32_t *__restrict__ eL,
-                            const int32_t *__restrict__ depth, const int32_t *__restrict__ tidx_of, const int4 *__restrict__ bot,
+                            const int32_t *__restrict__ depth, const int32_t *__restrict__ tidx_of, const int4 *__restrict__ bot, const uint8_t *__restrict__ row_of,
                             int n, int bits, int32_t lcap, const int32_t *__restrict__ eC, int2 *ex, int4 *eup,
                             int32_t *etr) {
   const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
@@ -1524,7 +1578,7 @@ __global__ void k_edge_refs(const int32_t *__restrict__ xoff, const int32_t *__r
     int ref = tidx_of[x];
     etr[e] = ref < 0 ? -1 : ref;
     if (ti < 0) {
-      if (x >= bt.x) ref = bt.z + (x - bt.x);
+      if (x >= bt.x) ref = row_of[x];
       else {  // a separator vertex of the bottom's root: its position in the root's list
         int lo = xoff[bt.x], hi = xoff[bt.x + 1];
         const int b0 = lo;
@@ -1671,12 +1725,23 @@ struct TreePlan {
   bool off = false;  // a count wrapped: the label kernels answer from now on
   std::vector<void *> owned;
 
+  char *arena = nullptr;  // one allocation for most arrays: each cudaMalloc and cudaFree costs a build ~0.1 ms
+  size_t arena_left = 0;
+
+  void *device(size_t size) {
+    void *p = nullptr;
+    CK(cudaMalloc(&p, size));
+    owned.push_back(p);
+    bytes += (int64_t)size;
+    return p;
+  }
   template <class T>
   T *alloc(size_t count) {
-    void *p = nullptr;
-    CK(cudaMalloc(&p, std::max<size_t>(count, 1) * sizeof(T)));
-    owned.push_back(p);
-    bytes += (int64_t)(std::max<size_t>(count, 1) * sizeof(T));
+    const size_t size = (std::max<size_t>(count, 1) * sizeof(T) + 255) & ~(size_t)255;
+    if (size > arena_left) return (T *)device(size);
+    char *p = arena;
+    arena += size;
+    arena_left -= size;
     return (T *)p;
   }
   template <class T>
@@ -1699,7 +1764,9 @@ void tree_free(DeviceState *d) {
 struct TreeShape {
   std::vector<int32_t> tidx_of;  // tid -> trunk index or -1 - bottom
   std::vector<int4> bot, piece;
-  std::vector<int32_t> piece_of, level_first, trunk_tid;
+  std::vector<uint8_t> row_of;   // tid in a bottom -> row, 0xff without descendants
+  std::vector<int32_t> piece_of, level_first, trunk_tid, chain_off;
+  std::vector<int2> chain;       // see TreeArgs
 };
 
 static TreeShape tree_shape(const Index &ix, const std::vector<int64_t> &soff) {
@@ -1709,17 +1776,23 @@ static TreeShape tree_shape(const Index &ix, const std::vector<int64_t> &soff) {
   std::vector<int32_t> heavy((size_t)n, -1), piece((size_t)n, -1);
   // bottoms: maximal subtrees whose separator and vertices fit the rows
   std::vector<char> is_bot((size_t)n, 0);
+  std::vector<int32_t> inner((size_t)n + 1, 0);  // vertices with descendants before t
+  for (int32_t t = 0; t < n; t++) inner[t + 1] = inner[t] + (ix.send[t] > t + 1);
+  s.row_of.assign((size_t)n, 0xff);
   for (int32_t t = 0; t < n;) {
-    const int32_t size = ix.send[t] - t, k = (int32_t)(soff[t + 1] - soff[t]);
-    if (size + k <= kBottomRows && soff[ix.send[t]] - soff[t] <= kBottomEdges) {
-      s.bot.push_back(make_int4(t, size, k, 0));
-      std::fill(is_bot.begin() + t, is_bot.begin() + ix.send[t], 1);
+    const int32_t size = ix.send[t] - t, k = (int32_t)(soff[t + 1] - soff[t]), rows = k + inner[ix.send[t]] - inner[t];
+    if (rows <= kBottomRows && size <= kBottomVerts && soff[ix.send[t]] - soff[t] <= kBottomEdges) {
+      s.bot.push_back(make_int4(t, size, k, rows));
+      for (int32_t x = t; x < ix.send[t]; x++) {
+        is_bot[x] = 1;
+        if (ix.send[x] > x + 1) s.row_of[x] = (uint8_t)(k + inner[x] - inner[t]);
+      }
       t = ix.send[t];
     } else {
       t++;
     }
   }
-  std::stable_sort(s.bot.begin(), s.bot.end(), [](const int4 &x, const int4 &y) { return x.y + x.z > y.y + y.z; });
+  std::stable_sort(s.bot.begin(), s.bot.end(), [](const int4 &x, const int4 &y) { return x.w > y.w; });
   for (size_t i = 0; i < s.bot.size(); i++)
     for (int32_t t = s.bot[i].x; t < s.bot[i].x + s.bot[i].y; t++) s.tidx_of[t] = -1 - (int32_t)i;
   // pieces: paths along the child with the largest subtree
@@ -1754,6 +1827,7 @@ static TreeShape tree_shape(const Index &ix, const std::vector<int64_t> &soff) {
   std::stable_sort(by_level.begin(), by_level.end(), [&](int32_t x, int32_t y) {
     return ps[x].level != ps[y].level ? ps[x].level < ps[y].level : ps[x].v.size() > ps[y].v.size();
   });
+  s.chain_off.assign(1, 0);
   for (int32_t id : by_level) {
     const int32_t first = (int32_t)s.trunk_tid.size(), np = (int32_t)s.piece.size();
     for (int32_t t : ps[id].v) {
@@ -1763,6 +1837,12 @@ static TreeShape tree_shape(const Index &ix, const std::vector<int64_t> &soff) {
     }
     const int32_t par = ix.parent[ps[id].v[0]];
     s.piece.push_back(make_int4(first, (int32_t)s.trunk_tid.size(), par < 0 ? -1 : s.tidx_of[par], 0));
+    if (par >= 0) {  // the parent's piece comes first, up to the parent itself
+      const int32_t pp = s.piece_of[s.tidx_of[par]], b = s.chain_off[pp], e = s.chain_off[pp + 1];
+      for (int32_t c = b; c < e; c++) s.chain.push_back(s.chain[c]);
+    }
+    s.chain.push_back(make_int2(first, ix.depth[ps[id].v[0]] - 1));
+    s.chain_off.push_back((int32_t)s.chain.size());
   }
   return s;
 }
@@ -1789,14 +1869,24 @@ void tree_build(Handle &h, DeviceState *d, const std::vector<int64_t> &soff, con
     return w * per_warp > (size_t)d->smem_optin - 2048 ? 0 : w;
   };
   const int up_warps = warps_for((size_t)H * 8);
-  if (!up_warps || (size_t)H * 20 + sizeof(BackShared) > (size_t)d->smem_optin - 2048) return;
+  if (!up_warps || (size_t)H * 20 + sizeof(BackShared<8>) > (size_t)d->smem_optin - 2048) return;
   cudaStream_t st = d->s_label;
   auto p = new TreePlan();
   d->tree = p;
   std::vector<void *> tmp;
-  auto talloc = [&](size_t bytes) {
+  // temporaries live in the per-source scratch, which no call uses yet, as far as it reaches
+  char *spare = reinterpret_cast<char *>(d->rec[0]);
+  size_t spare_left = (size_t)d->chunk * d->n_pad * sizeof(int4);
+  auto talloc = [&](size_t bytes) -> void * {
+    bytes = (std::max<size_t>(bytes, 16) + 255) & ~(size_t)255;
+    if (bytes <= spare_left) {
+      char *q = spare;
+      spare += bytes;
+      spare_left -= bytes;
+      return q;
+    }
     void *q = nullptr;
-    CK(cudaMalloc(&q, std::max<size_t>(bytes, 16)));
+    CK(cudaMalloc(&q, bytes));
     tmp.push_back(q);
     return q;
   };
@@ -1817,11 +1907,11 @@ void tree_build(Handle &h, DeviceState *d, const std::vector<int64_t> &soff, con
       }
       p->level_class.push_back(s.level_first[l + 1]);
     }
-    for (int i = 0; i < p->nbot;) {  // bottoms come largest first: launches of 32, 24, 16 and 8 rows
-      const int rows = (s.bot[i].y + s.bot[i].z + 7) & ~7;
+    for (int i = 0; i < p->nbot;) {  // bottoms come with the most rows first: a launch per four rows
+      auto rows_of = [&](int q) { return std::max(4, (s.bot[q].w + 3) & ~3); };
       int e = i;
-      while (e < p->nbot && ((s.bot[e].y + s.bot[e].z + 7) & ~7) == rows) e++;
-      p->bot_class.push_back({i, e, rows});
+      while (e < p->nbot && rows_of(e) == rows_of(i)) e++;
+      p->bot_class.push_back({i, e, rows_of(i)});
       i = e;
     }
     a.n = n;
@@ -1830,6 +1920,11 @@ void tree_build(Handle &h, DeviceState *d, const std::vector<int64_t> &soff, con
     a.bits = bits;
     a.dist_lim = (unsigned)(dmax + 1);
     a.absent = ((unsigned)(lim - 2 - dmax) << bits) | ((1u << bits) - 2u);
+    {
+      const size_t N = (size_t)n, T = s.trunk_tid.size(), e = (size_t)E;
+      p->arena_left = N * (4 + 4 + 1 + 8) + T * (16 + 8 + 4) + (s.piece.size() + s.bot.size()) * 16 + e * (8 + 4 + 4 + 4 + 16 + 24) + 64 * 256;
+      p->arena = (char *)p->device(p->arena_left);
+    }
     std::vector<int32_t> xoff(soff.begin(), soff.end());
     std::vector<int4> tmeta((size_t)a.NT);
     std::vector<int2> tsub((size_t)a.NT);
@@ -1844,8 +1939,11 @@ void tree_build(Handle &h, DeviceState *d, const std::vector<int64_t> &soff, con
     a.tsub = p->upload(tsub, st);
     a.piece = p->upload(s.piece, st);
     a.piece_of = p->upload(s.piece_of, st);
+    a.chain_off = p->upload(s.chain_off, st);
+    a.chain = p->upload(s.chain, st);
     a.tidx_of = p->upload(s.tidx_of, st);
     a.bot = p->upload(s.bot, st);
+    a.row_of = p->upload(s.row_of, st);
     a.depth = d->depth;
     a.parent = d->parent;
     a.send = d->send;
@@ -1881,7 +1979,7 @@ void tree_build(Handle &h, DeviceState *d, const std::vector<int64_t> &soff, con
       k_owner<<<blocks_for((int64_t)n * 32, 256), 256, 0, st>>>(a.xoff, n, owner);
       CK(cudaGetLastError());
       const int32_t lcap = (int32_t)(lim - 2 - dmax);
-      k_edge_refs<<<blocks_for((int64_t)n * 32, 256), 256, 0, st>>>(a.xoff, xtid, eL, d->depth, a.tidx_of, a.bot, n, bits, lcap, eC,
+      k_edge_refs<<<blocks_for((int64_t)n * 32, 256), 256, 0, st>>>(a.xoff, xtid, eL, d->depth, a.tidx_of, a.bot, a.row_of, n, bits, lcap, eC,
                                                                   ex, eup, etr);
       CK(cudaGetLastError());
       if (a.NT > 0) {
@@ -1989,21 +2087,21 @@ static size_t group_bytes(const TreeArgs &a) { return ((size_t)a.NT * (4 + 4 + 4
 constexpr int64_t kWideCtas = 148 * 12;  // (piece, group) pairs from which a level is wide
 
 // Groups of sources that the per-source scratch holds, at most kMaxGroups.
-constexpr int kMaxGroups = 128;
+constexpr int kMaxGroups = 1024;
 static int groups_fit(const DeviceState *d) {
   const size_t room = (size_t)d->chunk * d->n_pad * sizeof(int4);
   return (int)std::min<size_t>(kMaxGroups, room / group_bytes(d->tree->args));
 }
 
 // (source, vertex) pairs from which the tree is the faster path: its launches follow the trunk level by
-// level, about 1.1 ms at 50k vertices however few the sources, where the label kernels answer 16
-// sources in 1.07 ms and 64 in 1.38 ms, and 256 take 2.40 against 1.87 ms; 2,024 sources of 2,024
-// vertices 0.57 against 0.56 ms.  An H2H index's label path counts paths by Kahn waves (1.40 against
-// 0.60 ms there).  QBC_TREE_MIN_PAIRS overrides it for tests.
+// level, 0.8 to 1.1 ms at 50k vertices however few the sources, where the label kernels answer 1, 16,
+// 32, 64 sources in 0.52, 0.93, 1.02, 1.22 ms; at 6k vertices 128 sources take them 0.23 and the tree
+// 0.39 ms, 6,083 sources 3.15 and 1.20 ms.  An H2H index's label path counts paths by Kahn waves (2,024
+// sources of 2,024 vertices 1.40 and 0.47 ms).  QBC_TREE_MIN_PAIRS overrides it for tests.
 static int64_t min_pairs(const Handle &h) {
   const char *e = std::getenv("QBC_TREE_MIN_PAIRS");
   if (e && *e) return std::strtoll(e, nullptr, 10);
-  return h.host.kind == IndexKind::H2H ? (int64_t)1 << 20 : (int64_t)5 << 20;
+  return h.host.kind == IndexKind::H2H ? (int64_t)1 << 20 : (int64_t)2 << 20;
 }
 
 bool use_tree(const Handle &h, const DeviceState *d, int32_t ns) {
@@ -2016,6 +2114,16 @@ bool use_tree(const Handle &h, const DeviceState *d, int32_t ns) {
   const char *hook = std::getenv("QBC_TEST_ROW_WAIT_SPINS");
   if (hook && *hook) return false;
   return (int64_t)ns * d->n >= min_pairs(h) && groups_fit(d) >= 1;
+}
+
+bool tree_source_rows(const DeviceState *d, const int32_t *src, int32_t ns, int32_t stride, int32_t *rows, cudaStream_t st) {
+  if (!d->tree) return false;
+  TreeArgs a = d->tree->args;
+  a.src = src;
+  a.ns = ns;
+  k_source_rows<<<blocks_for((int64_t)ns * 32, 128), 128, 0, st>>>(a, stride, rows);
+  CK(cudaGetLastError());
+  return true;
 }
 
 const int32_t *tree_guard(const DeviceState *d) { return d->tree ? d->tree->args.wrap : nullptr; }
@@ -2044,7 +2152,9 @@ void launch_tree(const Handle &h, DeviceState *d, const int32_t *d_src_tid, int3
     CK(cudaGetLastError());
     d->launches++;
   };
-  const int fit = groups_fit(d);
+  // passes of equal size
+  const int groups = (ns + kGroup - 1) / kGroup, passes = (groups + groups_fit(d) - 1) / groups_fit(d);
+  const int fit = (groups + passes - 1) / passes;
   const int levels = (int)p.level_class.size() / 4;
   std::pair<cudaEvent_t, cudaEvent_t> ev{};
   for (int32_t off = 0; off < ns; off += fit * kGroup) {
@@ -2136,8 +2246,9 @@ void launch_tree(const Handle &h, DeviceState *d, const int32_t *d_src_tid, int3
     }
     {
       const size_t smem = (size_t)a.H * 20;
-      CK(cudaFuncSetAttribute(k_up_back, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      k_up_back<<<a.ns, kBackWarps * 32, smem, st>>>(a);
+      auto kern = a.ns >= 148 * 8 ? k_up_back<4> : k_up_back<8>;
+      CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      kern<<<a.ns, a.ns >= 148 * 8 ? 128 : 256, smem, st>>>(a);
       launched();
     }
     if (d->profiling) CK(cudaEventRecord(ev.second, st));
