@@ -60,7 +60,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
     os.makedirs(BUILD, exist_ok=True)
     os.makedirs(BIN, exist_ok=True)
     nvcc, cxx = _nvcc(), _cxx()
-    headers = [os.path.join(CSRC, h) for h in ("host.h", "device.h", "device_state.h")] + [os.path.join(INCLUDE, "qbc_b200.h")]
+    headers = [os.path.join(CSRC, h) for h in ("host.h", "device.h", "device_state.h", "frontier.cuh", "core.cuh")] + [os.path.join(INCLUDE, "qbc_b200.h")]
     objs = []
     for src, kind in (("host.cpp", "cxx"), ("index_file.cpp", "cxx"), ("capi.cpp", "cxx"), ("device.cu", "cu"), ("sssp.cu", "cu"), ("tree.cu", "cu"), ("sweep.cu", "cu")):
         s = os.path.join(CSRC, src)

@@ -2287,7 +2287,7 @@ static void launch_label(const Handle &h, DeviceState *d, int buf, const int32_t
       launch_sweep_rows_grid(h, d, d->rec[buf], d->hop[buf], d->order[buf], d->lcnt[buf], src, st);
     else
       launch_sweep_rows(h, d, d->rec[buf], d->hop[buf], d->order[buf], d->lcnt[buf], d->maxhop[buf], src, ns, st,
-                        need_hop);
+                        need_hop, guard);
     if (d->profiling) CK(cudaEventRecord(ev.second, st));
     d->label_launches++;
     d->launches++;
@@ -3248,6 +3248,7 @@ void device_upload(Handle &h, int device) {
       CK(cudaMemcpyAsync(d->ch, ix.ch.data(), ix.ch.size() * 4, cudaMemcpyHostToDevice, st));
     }
     finish_state(h, d);
+    if (ix.kind == IndexKind::CSR) core_build(h, d);
     if (!ix.seps.off.empty()) {  // (an index loaded from a file has none)
       int64_t *d_soff = nullptr;
       int4 *d_sep = nullptr;

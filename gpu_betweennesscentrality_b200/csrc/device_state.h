@@ -151,6 +151,7 @@ void launch_chunk(const Handle &h, DeviceState *d, const int32_t *d_src_tid, int
 void launch_sources(const Handle &h, DeviceState *d, const int32_t *d_src_tid, int32_t ns, cudaStream_t st, bool rerun);
 // BC over the elimination tree (tree.cu)
 void tree_build(Handle &h, DeviceState *d, const std::vector<int64_t> &soff, const int64_t *d_soff, const int4 *d_sep);
+void core_build(Handle &h, DeviceState *d);  // the same for the label-free index (core.cuh)
 void tree_free(DeviceState *d);
 bool use_tree(const Handle &h, const DeviceState *d, int32_t ns);
 // k_src_rows by the plan's runs of ancestors; false without a plan
@@ -165,7 +166,8 @@ void launch_tree(const Handle &h, DeviceState *d, const int32_t *d_src_tid, int3
 // write_hop false: hop layers are left out (the hop row is still the sweep's staging space); the
 // CTA pipelined dependency pass does not read them, it walks the wave queue.
 void launch_sweep_rows(const Handle &h, DeviceState *d, int4 *rec, int32_t *hop, int32_t *order, int32_t *lcnt,
-                       int32_t *maxhop, const int32_t *src, int32_t ns, cudaStream_t st, bool write_hop = true);
+                       int32_t *maxhop, const int32_t *src, int32_t ns, cudaStream_t st, bool write_hop = true,
+                       const int32_t *guard = nullptr);
 int32_t sweep_delta(const Handle &h, const DeviceState *d);
 // CSR index, plain path: one source's rows (slot 0 of a one-slot buffer; no largest-layer output)
 // by a cooperative launch of the whole GPU

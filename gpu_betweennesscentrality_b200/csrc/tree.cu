@@ -42,6 +42,7 @@
 #include <type_traits>
 
 #include "device_state.h"
+#include "frontier.cuh"
 
 namespace qbc {
 
@@ -1607,11 +1608,12 @@ __global__ void k_piece_edges(TreeArgs a, int4 *tmeta) {
   if (lane == 0) tmeta[i].z = c;
 }
 
-// triangles (y; t, x): shortcut (t, x) of least length through y.  A warp per (y, deeper vertex t).
+// triangles (y; t, x): shortcut (t, x) of least length through y.  A warp per (y, deeper vertex t),
+// from edge E0 on (the edges of a core before it are no eliminated vertex's).
 __global__ void k_triangles(const int32_t *__restrict__ xoff, const int32_t *__restrict__ xtid, const int32_t *__restrict__ eL,
-                            const int32_t *__restrict__ owner, int64_t E, int4 *tri, unsigned long long *count,
+                            const int32_t *__restrict__ owner, int64_t E0, int64_t E, int4 *tri, unsigned long long *count,
                             unsigned long long cap) {
-  const int64_t e2 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int64_t e2 = E0 + (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
   if (e2 >= E) return;
   const int y = owner[e2], first = xoff[y], t = xtid[e2], l2 = eL[e2];
@@ -1705,6 +1707,8 @@ __global__ void k_count_check(const double *__restrict__ cd, const int32_t *__re
 
 inline unsigned blocks_for(int64_t threads, int per) { return (unsigned)std::max<int64_t>(1, (threads + per - 1) / per); }
 
+#include "core.cuh"
+
 }  // namespace
 
 // Host part and device arrays of the plan.
@@ -1723,6 +1727,8 @@ struct TreePlan {
   int tail_level = 0;                // levels from here on hold at most kTailLevel triangles each
   int64_t E = 0, bytes = 0;
   bool off = false;  // a count wrapped: the label kernels answer from now on
+  CoreArgs core{};   // label-free index: nc > 0, without the scratch
+  const int32_t *cid_of = nullptr;
   std::vector<void *> owned;
 
   char *arena = nullptr;  // one allocation for most arrays: each cudaMalloc and cudaFree costs a build ~0.1 ms
@@ -1847,6 +1853,125 @@ static TreeShape tree_shape(const Index &ix, const std::vector<int64_t> &soff) {
   return s;
 }
 
+// Triangles of the edges [E0, E), level by level; false where their levels do not settle.
+template <class F>
+static bool build_triangles(TreePlan *p, int64_t E0, int64_t E, const int32_t *xtid, const int32_t *eL, F &&talloc, cudaStream_t st) {
+  const TreeArgs &a = p->args;
+  p->tri_first.assign(1, 0);
+  if (E0 >= E) return true;
+  int32_t *lvl = (int32_t *)talloc((size_t)E * 4), *flag = (int32_t *)talloc(16);
+  unsigned long long *cnt = (unsigned long long *)talloc(8 * (kMaxUnpackLevels + 2));
+  unsigned long long cap = (unsigned long long)E + 1024, found = 0;
+  int4 *raw = nullptr;
+  for (int round = 0; round < 2; round++) {
+    raw = (int4 *)talloc((size_t)cap * 16);
+    CK(cudaMemsetAsync(cnt, 0, 8, st));
+    k_triangles<<<blocks_for((E - E0) * 32, 256), 256, 0, st>>>(a.xoff, xtid, eL, p->owner, E0, E, raw, cnt, cap);
+    CK(cudaGetLastError());
+    CK(cudaMemcpyAsync(&found, cnt, 8, cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    if (found <= cap) break;
+    cap = found;
+  }
+  const int64_t T = (int64_t)found;
+  if (T == 0) return true;
+  CK(cudaMemsetAsync(lvl, 0, (size_t)E * 4, st));
+  bool settled = false;
+  for (int round = 0; round <= kMaxUnpackLevels && !settled; round += 4) {
+    int32_t ch = 0;
+    for (int q = 0; q < 4; q++) {
+      if (q == 3) CK(cudaMemsetAsync(flag, 0, 4, st));
+      k_levels<<<blocks_for(T, 256), 256, 0, st>>>(raw, T, lvl, flag);
+      CK(cudaGetLastError());
+    }
+    CK(cudaMemcpyAsync(&ch, flag, 4, cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    settled = ch == 0;
+  }
+  if (!settled) return false;
+  std::vector<unsigned long long> hist((size_t)kMaxUnpackLevels + 2, 0), first(1, 0);
+  CK(cudaMemsetAsync(cnt, 0, 8 * (kMaxUnpackLevels + 2), st));
+  k_level_hist<<<blocks_for(T, 256), 256, 0, st>>>(raw, T, lvl, cnt);
+  CK(cudaGetLastError());
+  CK(cudaMemcpyAsync(hist.data(), cnt, hist.size() * 8, cudaMemcpyDeviceToHost, st));
+  CK(cudaStreamSynchronize(st));
+  int32_t top = 0;
+  while (top < kMaxUnpackLevels && hist[top]) top++;
+  for (int l = 0; l < top; l++) {
+    p->tri_first.push_back(p->tri_first.back() + (int64_t)hist[l]);
+    first.push_back((unsigned long long)p->tri_first.back());
+  }
+  if (p->tri_first.back() != T) return false;
+  p->tri = p->alloc<int4>((size_t)T);
+  p->tri_at = p->upload(p->tri_first, st);
+  p->tail_level = top;
+  while (p->tail_level > 0 && hist[p->tail_level - 1] <= (unsigned long long)kTailLevel) p->tail_level--;
+  CK(cudaMemcpyAsync(cnt, first.data(), first.size() * 8, cudaMemcpyHostToDevice, st));
+  k_level_scatter<<<blocks_for(T, 256), 256, 0, st>>>(raw, T, lvl, cnt, p->tri);
+  CK(cudaGetLastError());
+  CK(cudaStreamSynchronize(st));  // the staging vectors die here
+  return true;
+}
+
+// Bottoms come with the most rows first: a launch per four rows.
+static void bottom_classes(TreePlan *p, const std::vector<int4> &bot) {
+  p->nbot = (int)bot.size();
+  for (int i = 0; i < p->nbot;) {
+    auto rows_of = [&](int q) { return std::max(4, (bot[q].w + 3) & ~3); };
+    int e = i;
+    while (e < p->nbot && rows_of(e) == rows_of(i)) e++;
+    p->bot_class.push_back({i, e, rows_of(i)});
+    i = e;
+  }
+}
+
+// Temporaries of a plan's build: in the per-source scratch, which no call uses yet, as far as it
+// reaches, else on their own.
+struct PlanScratch {
+  char *spare;
+  size_t left;
+  std::vector<void *> own;
+  explicit PlanScratch(DeviceState *d)
+      : spare(reinterpret_cast<char *>(d->rec[0])), left((size_t)d->chunk * d->n_pad * sizeof(int4)) {}
+  ~PlanScratch() {
+    for (void *q : own) cudaFree(q);
+  }
+  void *operator()(size_t bytes) {
+    bytes = (std::max<size_t>(bytes, 16) + 255) & ~(size_t)255;
+    if (bytes <= left) {
+      char *q = spare;
+      spare += bytes;
+      left -= bytes;
+      return q;
+    }
+    void *q = nullptr;
+    CK(cudaMalloc(&q, bytes));
+    own.push_back(q);
+    return q;
+  }
+};
+
+// The plan is the index's now, or gone.
+static void plan_done(DeviceState *d, bool keep) {
+  if (keep) {
+    d->bytes += d->tree->bytes;
+  } else {
+    d->tree->bytes = 0;
+    tree_free(d);
+  }
+}
+
+// After an exception in a build: no room for the plan means that the general kernels answer.
+static void plan_failed(DeviceState *d) {
+  plan_done(d, false);
+  try {
+    throw;
+  } catch (const Error &e) {
+    if (e.code != QBC_ENOMEM) throw;
+    cudaGetLastError();
+  }
+}
+
 // Builds the plan from the separators (soff on the host; d_soff / d_sep their device copies).  The
 // plan is left out, and the label kernels keep answering, where its keys do not fit 32 bits, a
 // shortcut count has wrapped, a row does not fit shared memory, or memory is short.
@@ -1873,23 +1998,7 @@ void tree_build(Handle &h, DeviceState *d, const std::vector<int64_t> &soff, con
   cudaStream_t st = d->s_label;
   auto p = new TreePlan();
   d->tree = p;
-  std::vector<void *> tmp;
-  // temporaries live in the per-source scratch, which no call uses yet, as far as it reaches
-  char *spare = reinterpret_cast<char *>(d->rec[0]);
-  size_t spare_left = (size_t)d->chunk * d->n_pad * sizeof(int4);
-  auto talloc = [&](size_t bytes) -> void * {
-    bytes = (std::max<size_t>(bytes, 16) + 255) & ~(size_t)255;
-    if (bytes <= spare_left) {
-      char *q = spare;
-      spare += bytes;
-      spare_left -= bytes;
-      return q;
-    }
-    void *q = nullptr;
-    CK(cudaMalloc(&q, bytes));
-    tmp.push_back(q);
-    return q;
-  };
+  PlanScratch talloc(d);
   bool keep = false;
   try {
     TreeArgs &a = p->args;
@@ -1897,7 +2006,6 @@ void tree_build(Handle &h, DeviceState *d, const std::vector<int64_t> &soff, con
     p->up_warps = up_warps;
     const int32_t n = ix.n;
     const TreeShape s = tree_shape(ix, soff);
-    p->nbot = (int)s.bot.size();
     for (size_t l = 0; l + 1 < s.level_first.size(); l++) {  // (longest first, see tree_shape)
       int32_t q = s.level_first[l];
       p->level_class.push_back(q);
@@ -1907,13 +2015,7 @@ void tree_build(Handle &h, DeviceState *d, const std::vector<int64_t> &soff, con
       }
       p->level_class.push_back(s.level_first[l + 1]);
     }
-    for (int i = 0; i < p->nbot;) {  // bottoms come with the most rows first: a launch per four rows
-      auto rows_of = [&](int q) { return std::max(4, (s.bot[q].w + 3) & ~3); };
-      int e = i;
-      while (e < p->nbot && rows_of(e) == rows_of(i)) e++;
-      p->bot_class.push_back({i, e, rows_of(i)});
-      i = e;
-    }
+    bottom_classes(p, s.bot);
     a.n = n;
     a.H = H;
     a.NT = (int)s.trunk_tid.size();
@@ -1969,9 +2071,7 @@ void tree_build(Handle &h, DeviceState *d, const std::vector<int64_t> &soff, con
     a.wrap = d->err + 1;
     CK(cudaMemsetAsync(a.wrap, 0, 4, st));
     int32_t *xtid = (int32_t *)talloc((size_t)E * 4), *eL = (int32_t *)talloc((size_t)E * 4);
-    int32_t *lvl = (int32_t *)talloc((size_t)E * 4);
     double *cd = a.Bd;  // the edge accumulators are free until the first call
-    unsigned long long *cnt = (unsigned long long *)talloc(8 * (kMaxUnpackLevels + 2));
     int32_t *flag = (int32_t *)talloc(16);
     if (E > 0) {
       k_sort_edges<<<blocks_for((int64_t)n * 32, 256), 256, 0, st>>>(d_soff, d_sep, n, xtid, eL, eC);
@@ -1986,59 +2086,8 @@ void tree_build(Handle &h, DeviceState *d, const std::vector<int64_t> &soff, con
         k_piece_edges<<<blocks_for((int64_t)a.NT * 32, 256), 256, 0, st>>>(a, tm);
         CK(cudaGetLastError());
       }
-      // triangles
-      unsigned long long cap = (unsigned long long)E + 1024, found = 0;
-      int4 *raw = nullptr;
-      for (int round = 0; round < 2; round++) {
-        raw = (int4 *)talloc((size_t)cap * 16);
-        CK(cudaMemsetAsync(cnt, 0, 8, st));
-        k_triangles<<<blocks_for(E * 32, 256), 256, 0, st>>>(a.xoff, xtid, eL, owner, E, raw, cnt, cap);
-        CK(cudaGetLastError());
-        CK(cudaMemcpyAsync(&found, cnt, 8, cudaMemcpyDeviceToHost, st));
-        CK(cudaStreamSynchronize(st));
-        if (found <= cap) break;
-        cap = found;
-      }
-      const int64_t T = (int64_t)found;
-      CK(cudaMemsetAsync(lvl, 0, (size_t)E * 4, st));
-      int32_t top = 0;
-      bool settled = T == 0;
-      for (int round = 0; round <= kMaxUnpackLevels && !settled; round += 4) {
-        int32_t ch = 0;
-        for (int q = 0; q < 4; q++) {
-          if (q == 3) CK(cudaMemsetAsync(flag, 0, 4, st));
-          k_levels<<<blocks_for(T, 256), 256, 0, st>>>(raw, T, lvl, flag);
-          CK(cudaGetLastError());
-        }
-        CK(cudaMemcpyAsync(&ch, flag, 4, cudaMemcpyDeviceToHost, st));
-        CK(cudaStreamSynchronize(st));
-        settled = ch == 0;
-      }
-      if (settled) {
-        std::vector<unsigned long long> hist((size_t)kMaxUnpackLevels + 2, 0), first;
-        CK(cudaMemsetAsync(cnt, 0, 8 * (kMaxUnpackLevels + 2), st));
-        if (T > 0) {
-          k_level_hist<<<blocks_for(T, 256), 256, 0, st>>>(raw, T, lvl, cnt);
-          CK(cudaGetLastError());
-        }
-        CK(cudaMemcpyAsync(hist.data(), cnt, hist.size() * 8, cudaMemcpyDeviceToHost, st));
-        CK(cudaStreamSynchronize(st));
-        while (top < kMaxUnpackLevels && hist[top]) top++;
-        p->tri_first.assign(1, 0);
-        first.push_back(0);
-        for (int l = 0; l < top; l++) {
-          p->tri_first.push_back(p->tri_first.back() + (int64_t)hist[l]);
-          first.push_back((unsigned long long)p->tri_first.back());
-        }
-        p->tri = p->alloc<int4>((size_t)T);
-        p->tri_at = p->upload(p->tri_first, st);
-        p->tail_level = top;
-        while (p->tail_level > 0 && hist[p->tail_level - 1] <= (unsigned long long)kTailLevel) p->tail_level--;
-        CK(cudaMemcpyAsync(cnt, first.data(), first.size() * 8, cudaMemcpyHostToDevice, st));
-        if (T > 0) {
-          k_level_scatter<<<blocks_for(T, 256), 256, 0, st>>>(raw, T, lvl, cnt, p->tri);
-          CK(cudaGetLastError());
-        }
+      if (build_triangles(p, 0, E, xtid, eL, talloc, st)) {
+        const int top = (int)p->tri_first.size() - 1;
         k_count_arcs<<<blocks_for(E, 256), 256, 0, st>>>(owner, xtid, eL, E, d->arc_rng, d->arc_hw, cd);
         CK(cudaGetLastError());
         for (int l = top - 1; l >= 0; l--) {
@@ -2052,7 +2101,7 @@ void tree_build(Handle &h, DeviceState *d, const std::vector<int64_t> &soff, con
         CK(cudaGetLastError());
         CK(cudaMemcpyAsync(&bad, flag, 4, cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
-        keep = bad == 0 && p->tri_first.back() == T;
+        keep = bad == 0;
       }
     } else {
       p->tri_first.assign(1, 0);
@@ -2060,29 +2109,105 @@ void tree_build(Handle &h, DeviceState *d, const std::vector<int64_t> &soff, con
     }
     CK(cudaStreamSynchronize(st));  // the staging vectors die here
   } catch (...) {
-    for (void *q : tmp) cudaFree(q);
-    p->bytes = 0;  // not yet part of the index's
-    tree_free(d);
-    try {
-      throw;
-    } catch (const Error &e) {
-      if (e.code != QBC_ENOMEM) throw;
-      cudaGetLastError();  // no room for the plan: the label kernels answer
+    return plan_failed(d);
+  }
+  plan_done(d, keep);
+}
+
+// The same for the label-free index (see core.cuh): its plan keeps keys of lengths below lim, of which
+// a core distance may take a quarter (checked at each sweep) and a bottom's chain another.
+void core_build(Handle &h, DeviceState *d) {
+  NvtxRange nvtx("qbc.core_plan");
+  TraceScope trace("core plan");
+  const Index &ix = h.host;
+  tree_free(d);
+  const int32_t n = ix.n;
+  constexpr int bits = 5;
+  static_assert(kBottomRows + 1 < (1 << bits) - 2, "entry index");
+  constexpr uint32_t lim = 1u << (32 - bits);
+  const int32_t lcap = (int32_t)(lim / (4 * kCoreChain));
+  CoreShape s;
+  if (!core_shape(ix, s) || (int64_t)s.nc * 4 > (int64_t)n * 3) return;  // (a core that is most of the graph saves nothing)
+  if ((size_t)core_words(s.nc) * 8 + 8192 > (size_t)d->smem_optin) return;  // its list bits are in shared memory
+  for (size_t e = (size_t)s.xoff[s.nc]; e < s.eL.size(); e++)
+    if (s.eL[e] > lcap) return;
+  cudaStream_t st = d->s_label;
+  auto p = new TreePlan();
+  d->tree = p;
+  bool keep = false;
+  try {
+    PlanScratch talloc(d);
+    TreeArgs &a = p->args;
+    const int64_t E = (int64_t)s.xtid.size(), E0 = s.xoff[s.nc];
+    p->E = E;
+    bottom_classes(p, s.bot);
+    a.n = n;
+    a.H = kCoreH;
+    a.NT = s.nc;
+    a.bits = bits;
+    a.dist_lim = lim / 4;
+    a.absent = ((lim / 10 * 7) << bits) | ((1u << bits) - 2u);
+    p->arena_left = (size_t)n * (7 * 4 + 1 + 8) + s.bot.size() * 16 + (size_t)E * (8 + 4 + 4 + 4 + 16 + 24) +
+                    (s.arc.size() * 2 + s.more.size()) * 16 + 64 * 256;
+    p->arena = (char *)p->device(p->arena_left);
+    a.xoff = p->upload(s.xoff, st);
+    a.tidx_of = p->upload(s.tidx_of, st);
+    a.bot = p->upload(s.bot, st);
+    a.row_of = p->upload(s.row_of, st);
+    a.depth = p->upload(s.depth, st);
+    a.parent = p->upload(s.parent, st);
+    a.send = p->upload(s.send, st);
+    p->cid_of = p->upload(s.cid_of, st);
+    int32_t *eC = p->upload(s.eC, st);
+    CoreArgs &c = p->core;
+    c.nc = s.nc;
+    c.arc = p->upload(s.arc, st);
+    c.info = p->upload(s.info, st);
+    c.more = p->upload(s.more, st);
+    c.E = E;
+    c.max_rounds = 2 * s.nc + 16;
+    while (((s.nc - 1) >> c.sort_shift) >= kCoreBuckets) c.sort_shift++;
+    c.sort_buckets = ((s.nc - 1) >> c.sort_shift) + 1;
+    int2 *ex = p->alloc<int2>((size_t)E);
+    int4 *eup = p->alloc<int4>((size_t)E);
+    int32_t *etr = p->alloc<int32_t>((size_t)E);
+    p->owner = p->alloc<int32_t>((size_t)E);
+    a.ex = ex;
+    a.eC = eC;
+    a.eup = eup;
+    a.etr = etr;
+    a.Bd = p->alloc<double>((size_t)E * 3 + (size_t)n);
+    a.Bu = a.Bd + E;
+    a.Bs = a.Bu + E;
+    a.F = a.Bs + E;
+    a.wrap = d->err + 1;
+    CK(cudaMemsetAsync(a.wrap, 0, 4, st));
+    int32_t *xtid = (int32_t *)talloc((size_t)E * 4), *eL = (int32_t *)talloc((size_t)E * 4);
+    if (E > 0) {
+      CK(cudaMemcpyAsync(xtid, s.xtid.data(), (size_t)E * 4, cudaMemcpyHostToDevice, st));
+      CK(cudaMemcpyAsync(eL, s.eL.data(), (size_t)E * 4, cudaMemcpyHostToDevice, st));
+      k_owner<<<blocks_for((int64_t)n * 32, 256), 256, 0, st>>>(a.xoff, n, p->owner);
+      CK(cudaGetLastError());
+      k_edge_refs<<<blocks_for((int64_t)n * 32, 256), 256, 0, st>>>(a.xoff, xtid, eL, a.depth, a.tidx_of, a.bot, a.row_of, n, bits,
+                                                                  lcap, eC, ex, eup, etr);
+      CK(cudaGetLastError());
     }
-    return;
+    keep = build_triangles(p, E0, E, xtid, eL, talloc, st);
+    CK(cudaStreamSynchronize(st));  // the staging vectors die here
+  } catch (...) {
+    return plan_failed(d);
   }
-  for (void *q : tmp) cudaFree(q);
-  if (keep) {
-    d->bytes += p->bytes;
-  } else {
-    p->bytes = 0;
-    tree_free(d);
-  }
+  plan_done(d, keep);
 }
 
 // ------------------------------------------------------------------------------- launch
 // device bytes of one group of sources
-static size_t group_bytes(const TreeArgs &a) { return ((size_t)a.NT * (4 + 4 + 4 + 8) + (size_t)a.H * (4 + 4 + 8)) * kGroup; }
+static size_t group_bytes(const TreePlan &p) {
+  const TreeArgs &a = p.args;
+  if (p.core.nc)  // sweep state, rows of D, S and J, rows of U and the seeds, source and waves
+    return ((size_t)a.NT * (4 + 8 + 4 + 4 + 8) + (size_t)a.H * (4 + 4 + 8) + 8) * kGroup;
+  return ((size_t)a.NT * (4 + 4 + 4 + 8) + (size_t)a.H * (4 + 4 + 8)) * kGroup;
+}
 
 constexpr int64_t kWideCtas = 148 * 12;  // (piece, group) pairs from which a level is wide
 
@@ -2090,7 +2215,10 @@ constexpr int64_t kWideCtas = 148 * 12;  // (piece, group) pairs from which a le
 constexpr int kMaxGroups = 1024;
 static int groups_fit(const DeviceState *d) {
   const size_t room = (size_t)d->chunk * d->n_pad * sizeof(int4);
-  return (int)std::min<size_t>(kMaxGroups, room / group_bytes(d->tree->args));
+  size_t fit = std::min<size_t>(kMaxGroups, room / group_bytes(*d->tree));
+  if (d->tree->core.nc)  // the lists of a core vertex take the place of a vertex's
+    fit = std::min<size_t>(fit, (size_t)d->chunk * d->n_pad / ((size_t)(d->tree->core.nc + 2) * kGroup));
+  return (int)fit;
 }
 
 // (source, vertex) pairs from which the tree is the faster path: its launches follow the trunk level by
@@ -2101,6 +2229,7 @@ static int groups_fit(const DeviceState *d) {
 static int64_t min_pairs(const Handle &h) {
   const char *e = std::getenv("QBC_TREE_MIN_PAIRS");
   if (e && *e) return std::strtoll(e, nullptr, 10);
+  if (h.host.kind == IndexKind::CSR) return 0;  // (one source of 100 vertices 0.146 against 0.170 ms)
   return h.host.kind == IndexKind::H2H ? (int64_t)1 << 20 : (int64_t)2 << 20;
 }
 
@@ -2117,7 +2246,7 @@ bool use_tree(const Handle &h, const DeviceState *d, int32_t ns) {
 }
 
 bool tree_source_rows(const DeviceState *d, const int32_t *src, int32_t ns, int32_t stride, int32_t *rows, cudaStream_t st) {
-  if (!d->tree) return false;
+  if (!d->tree || d->tree->core.nc) return false;
   TreeArgs a = d->tree->args;
   a.src = src;
   a.ns = ns;
@@ -2145,7 +2274,139 @@ static void launch_bottom(const TreeArgs &a, int first, int end, int rows, cudaS
   k_bottom<<<dim3(end - first, (a.ng + gpc - 1) / gpc), warps * 32, smem, st>>>(a, first, rows, gpc);
 }
 
+static void launch_bottoms(DeviceState *d, const TreeArgs &a, cudaStream_t st) {
+  const TreePlan &p = *d->tree;
+  if (a.ng > 4) {
+    for (const TreePlan::BotClass &c : p.bot_class) {
+      launch_bottom(a, c.first, c.end, c.rows, st);
+      CK(cudaGetLastError());
+      d->launches++;
+    }
+  } else if (p.nbot) {
+    launch_bottom(a, 0, p.nbot, p.bot_class[0].rows, st);
+    CK(cudaGetLastError());
+    d->launches++;
+  }
+}
+
+// B over the triangles, into F
+static void launch_unpack(DeviceState *d, cudaStream_t st) {
+  const TreePlan &p = *d->tree;
+  const TreeArgs &a = p.args;
+  auto launched = [&] {
+    CK(cudaGetLastError());
+    d->launches++;
+  };
+  if (p.E > 0) {
+    k_fold<<<blocks_for(p.E, 256), 256, 0, st>>>(p.E, a.eup, p.owner, a.Bd, a.Bu, a.Bs, a.F, a.wrap);
+    launched();
+  }
+  const int top = (int)p.tri_first.size() - 1;
+  for (int l = 0; l < p.tail_level; l++) {
+    const int64_t b = p.tri_first[l], c = p.tri_first[l + 1] - b;
+    k_unpack<<<blocks_for(c, 256), 256, 0, st>>>(p.tri + b, c, a.eC, a.Bd, a.F, a.wrap);
+    launched();
+  }
+  if (p.tail_level < top) {
+    k_unpack_tail<<<1, 1024, 0, st>>>(p.tri, p.tri_at, p.tail_level, top, a.eC, a.Bd, a.F, a.wrap);
+    launched();
+  }
+}
+
+// Threads per CTA of the core's sweep and dependencies; 2,048 per SM in any case.
+static int core_threads(const Handle &h, int ns, int nc) {
+  const int t = h.tuning.sweep_threads;
+  if (t) return t == 2048 ? 512 : t;
+  if (ns <= 148 * 2 || nc >= kCoreLarge) return 1024;
+  return ns > 148 * 4 && nc < kCoreSmall ? 256 : 512;
+}
+struct CoreKernels {
+  void (*sweep)(TreeArgs, CoreArgs), (*dep)(TreeArgs, CoreArgs);
+};
+static CoreKernels core_kernels(int threads) {
+  switch (threads) {
+    case 256: return {k_core_sweep<256, 8>, k_core_dep<256, 8>};
+    case 512: return {k_core_sweep<512, 4>, k_core_dep<512, 4>};
+    default: return {k_core_sweep<1024, 2>, k_core_dep<1024, 2>};
+  }
+}
+
+// The label-free index: sweeps over the core, bottoms, dependencies over the core (see core.cuh).
+static void launch_core(const Handle &h, DeviceState *d, const int32_t *d_src_tid, int32_t ns, cudaStream_t st) {
+  TreePlan &p = *d->tree;
+  const int32_t nc = p.core.nc;
+  CK(cudaMemsetAsync(p.args.Bd, 0, ((size_t)p.E * 3 + (size_t)p.args.n) * 8, st));
+  auto launched = [&] {
+    CK(cudaGetLastError());
+    d->launches++;
+  };
+  const int groups = (ns + kGroup - 1) / kGroup, passes = (groups + groups_fit(d) - 1) / groups_fit(d);
+  const int fit = (groups + passes - 1) / passes;
+  std::pair<cudaEvent_t, cudaEvent_t> ev{};
+  for (int32_t off = 0; off < ns; off += fit * kGroup) {
+    TreeArgs a = p.args;
+    CoreArgs c = p.core;
+    a.ns = std::min(fit * kGroup, ns - off);
+    a.ng = (a.ns + kGroup - 1) / kGroup;
+    const size_t slots = (size_t)a.ng * kGroup, nt = slots * nc, nu = slots * a.H;
+    char *w = reinterpret_cast<char *>(d->rec[0]);
+    auto take = [&](size_t bytes) {
+      char *q = w;
+      w += bytes;
+      return q;
+    };
+    c.word = (unsigned long long *)take(nt * 8);
+    a.J = (double *)take(nt * 8);
+    a.seed = (double *)take(nu * 8);
+    a.D = (uint32_t *)take(nt * 4);
+    a.S = (uint32_t *)take(nt * 4);
+    a.Ud = (int32_t *)take(nu * 4);
+    a.Uc = (uint32_t *)take(nu * 4);
+    int32_t *cid = (int32_t *)take(slots * 4);
+    c.waves = (int32_t *)take(slots * 4);
+    c.dist = (int32_t *)take(nt * 4);
+    a.src = cid;
+    c.hop = d->hop[0];
+    c.order = d->order[0];
+    c.lcnt = d->lcnt[0];
+    c.delta = sweep_delta(h, d) * kCoreDelta;
+    const int threads = core_threads(h, a.ns, nc);
+    const CoreKernels kernels = core_kernels(threads);
+    const size_t smem = (size_t)core_words(nc) * 8;
+    CK(cudaFuncSetAttribute(kernels.sweep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (d->profiling) {
+      ev = take_events(d->ev_lab, d->ev_lab_used);
+      CK(cudaEventRecord(ev.first, st));
+    }
+    k_core_src<<<blocks_for(a.ns, 256), 256, 0, st>>>(d_src_tid + off, p.cid_of, a.ns, cid);
+    launched();
+    k_core_up<<<(unsigned)(slots / 4), 128, 0, st>>>(a);
+    launched();
+    kernels.sweep<<<a.ns, threads, smem, st>>>(a, c);
+    launched();
+    k_core_rows<<<dim3((nc + 31) / 32, a.ng), 256, 0, st>>>(a, c);
+    launched();
+    launch_bottoms(d, a, st);
+    if (d->profiling) {
+      CK(cudaEventRecord(ev.second, st));
+      ev = take_events(d->ev_dp, d->ev_dp_used);
+      CK(cudaEventRecord(ev.first, st));
+    }
+    kernels.dep<<<a.ns, threads, 0, st>>>(a, c);
+    launched();
+    k_core_back<<<blocks_for(a.ns, 4), 128, 0, st>>>(a, c);
+    launched();
+    if (d->profiling) CK(cudaEventRecord(ev.second, st));
+    d->label_launches++;
+    d->dep_launches++;
+  }
+  launch_unpack(d, st);
+  k_core_finish<<<blocks_for(p.args.n, 256), 256, 0, st>>>(p.args.F, p.cid_of, d->bc_tid, p.args.n, p.args.wrap);
+  launched();
+}
+
 void launch_tree(const Handle &h, DeviceState *d, const int32_t *d_src_tid, int32_t ns, cudaStream_t st) {
+  if (d->tree->core.nc) return launch_core(h, d, d_src_tid, ns, st);
   TreePlan &p = *d->tree;
   CK(cudaMemsetAsync(p.args.Bd, 0, ((size_t)p.E * 3 + (size_t)p.args.n) * 8, st));
   auto launched = [&] {
@@ -2210,15 +2471,7 @@ void launch_tree(const Handle &h, DeviceState *d, const int32_t *d_src_tid, int3
         launched();
       }
     }
-    if (a.ng > 4) {
-      for (const TreePlan::BotClass &c : p.bot_class) {
-        launch_bottom(a, c.first, c.end, c.rows, st);
-        launched();
-      }
-    } else if (p.nbot) {
-      launch_bottom(a, 0, p.nbot, p.bot_class[0].rows, st);
-      launched();
-    }
+    launch_bottoms(d, a, st);
     if (d->profiling) {
       CK(cudaEventRecord(ev.second, st));
       ev = take_events(d->ev_dp, d->ev_dp_used);
@@ -2255,21 +2508,7 @@ void launch_tree(const Handle &h, DeviceState *d, const int32_t *d_src_tid, int3
     d->label_launches++;
     d->dep_launches++;
   }
-  const TreeArgs &a = p.args;
-  if (p.E > 0) {
-    k_fold<<<blocks_for(p.E, 256), 256, 0, st>>>(p.E, a.eup, p.owner, a.Bd, a.Bu, a.Bs, a.F, a.wrap);
-    launched();
-  }
-  const int top = (int)p.tri_first.size() - 1;
-  for (int l = 0; l < p.tail_level; l++) {
-    const int64_t b = p.tri_first[l], c = p.tri_first[l + 1] - b;
-    k_unpack<<<blocks_for(c, 256), 256, 0, st>>>(p.tri + b, c, a.eC, a.Bd, a.F, a.wrap);
-    launched();
-  }
-  if (p.tail_level < top) {
-    k_unpack_tail<<<1, 1024, 0, st>>>(p.tri, p.tri_at, p.tail_level, top, a.eC, a.Bd, a.F, a.wrap);
-    launched();
-  }
+  launch_unpack(d, st);
   k_finish<<<std::min(148 * 4, (p.args.n + 255) / 256), 256, 0, st>>>(p.args.F, d->bc_tid, p.args.n, p.args.wrap);
   launched();
 }
