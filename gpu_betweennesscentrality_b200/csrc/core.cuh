@@ -509,6 +509,26 @@ __global__ void k_core_finish(const double *__restrict__ F, const int32_t *__res
 }
 
 // ------------------------------------------------------------------------------- plan
+// f(begin, end) over ranges of [0, count) on a few threads; f does not throw
+template <class F>
+static void core_ranges(int32_t count, F &&f) {
+  const int nt = count < 20000 ? 1 : (int)std::min(8u, std::max(1u, std::thread::hardware_concurrency()));
+  std::vector<std::thread> ts;
+  ts.reserve((size_t)nt);
+  for (int t = 0; t < nt; t++) {
+    const int32_t b = (int32_t)((int64_t)count * t / nt), e = (int32_t)((int64_t)count * (t + 1) / nt);
+    if (t + 1 < nt) {
+      try {
+        ts.emplace_back([&f, b, e] { f(b, e); });
+        continue;
+      } catch (const std::system_error &) {  // no thread to be had
+      }
+    }
+    f(b, e);
+  }
+  for (std::thread &t : ts) t.join();
+}
+
 // The elimination; false where no plan is possible (a count past 2^31, a degree past the sweep's, or
 // lengths below 1, which a graph has none of but a file might).
 static bool core_shape(const Index &ix, CoreShape &s) {
@@ -520,29 +540,33 @@ static bool core_shape(const Index &ix, CoreShape &s) {
     int64_t off;
     int32_t len, cap;
   };
+  // lists with room for one more entry each; a list that grows past its room moves to the end
   std::vector<List> adj((size_t)n);
-  std::vector<Ent> pool((size_t)ix.arc_off[n] + (size_t)n);
-  pool.reserve(pool.size() * 2);
-  int64_t at = 0;
-  for (int32_t v = 0; v < n; v++) {
-    const int32_t b = ix.arc_off[v], e = ix.arc_off[v + 1];
-    adj[v] = {at, e - b, e - b + 1};
-    for (int32_t q = b; q < e; q++) {
-      if (ix.arc_w[q] < 1) return false;
-      pool[at + q - b] = {ix.arc_head[q], ix.arc_w[q], 1};
+  int64_t room = 2 * ((int64_t)ix.arc_off[n] + n), used = (int64_t)ix.arc_off[n] + n;
+  std::unique_ptr<Ent[]> pool(new Ent[(size_t)room]);
+  std::atomic<bool> ok{true};
+  core_ranges(n, [&](int32_t v0, int32_t v1) {
+    for (int32_t v = v0; v < v1; v++) {
+      const int32_t b = ix.arc_off[v], e = ix.arc_off[v + 1];
+      adj[v] = {(int64_t)b + v, e - b, e - b + 1};
+      for (int32_t q = b; q < e; q++) {
+        if (ix.arc_w[q] < 1) ok = false;
+        pool[(int64_t)q + v] = {ix.arc_head[q], ix.arc_w[q], 1};
+      }
     }
-    at += e - b + 1;
-  }
+  });
+  if (!ok) return false;
   auto find = [&](int32_t u, int32_t h) {
     for (int32_t q = 0; q < adj[u].len; q++)
       if (pool[adj[u].off + q].h == h) return q;
     return -1;
   };
   // eliminated vertices: entries, state of the subtree; pending roots per live vertex (4 links each)
-  std::vector<Ent> xs((size_t)n * kCoreDegree);
+  std::unique_ptr<Ent[]> xs(new Ent[(size_t)n * kCoreDegree]);
   std::vector<int8_t> nx((size_t)n, -1);  // entries of an eliminated vertex; -1 live, -2 live for good
   std::vector<uint8_t> size((size_t)n, 0), inner((size_t)n, 0), edges((size_t)n, 0);
-  std::vector<int32_t> up((size_t)n, -1), head((size_t)n, -1), link((size_t)n * kCoreDegree, -1);
+  std::vector<int32_t> up((size_t)n, -1), head((size_t)n, -1);
+  std::unique_ptr<int32_t[]> link(new int32_t[(size_t)n * kCoreDegree]);
   std::vector<std::vector<int32_t>> bucket(kCoreDegree + 1);
   for (int32_t v = n - 1; v >= 0; v--)
     if (adj[v].len >= 1 && adj[v].len <= kCoreDegree) bucket[adj[v].len].push_back(v);
@@ -578,7 +602,7 @@ static bool core_shape(const Index &ix, CoreShape &s) {
     inner[v] = (uint8_t)in;
     edges[v] = (uint8_t)ed;
     nx[v] = (int8_t)k;
-    Ent *x = xs.data() + (size_t)v * kCoreDegree;
+    Ent *x = xs.get() + (size_t)v * kCoreDegree;
     for (int i = 0; i < k; i++) {
       x[i] = pool[adj[v].off + i];
       link[(size_t)v * kCoreDegree + i] = head[x[i].h];
@@ -596,11 +620,16 @@ static bool core_shape(const Index &ix, CoreShape &s) {
         if (q < 0) {
           if (C > INT_MAX) return false;
           if (a.len == a.cap) {
-            const int64_t off = (int64_t)pool.size();
-            pool.resize(pool.size() + 2 * a.cap);
-            std::copy(pool.begin() + a.off, pool.begin() + a.off + a.len, pool.begin() + off);
-            a.off = off;
+            if (used + 2 * a.cap > room) {
+              room = 2 * room + 2 * a.cap;
+              std::unique_ptr<Ent[]> larger(new Ent[(size_t)room]);
+              std::copy(pool.get(), pool.get() + used, larger.get());
+              pool.swap(larger);
+            }
+            std::copy(pool.get() + a.off, pool.get() + a.off + a.len, pool.get() + used);
+            a.off = used;
             a.cap *= 2;
+            used += a.cap;
           }
           pool[a.off + a.len++] = {x[j].h, L, (int32_t)C};
         } else {
@@ -667,54 +696,69 @@ static bool core_shape(const Index &ix, CoreShape &s) {
   for (int32_t i = 0; i < s.nbot; i++)
     for (int32_t c = s.bot[i].x; c < s.bot[i].x + s.bot[i].y; c++) s.tidx_of[c] = -1 - i;
   // edges, then the core's arcs
+  auto list_of = [&](int32_t t) { return nx[t] < 0 ? pool.get() + adj[t].off : xs.get() + (size_t)t * kCoreDegree; };
+  auto length_of = [&](int32_t t) { return nx[t] < 0 ? adj[t].len : (int32_t)nx[t]; };
   s.xoff.assign((size_t)n + 1, 0);
-  std::vector<Ent> list;
-  std::vector<int64_t> core_place;
-  for (int32_t c = 0; c < n; c++) {
-    const int32_t t = s.tid_of[c];
-    list.clear();
-    const Ent *x = nx[t] < 0 ? pool.data() + adj[t].off : xs.data() + (size_t)t * kCoreDegree;
-    const int32_t k = nx[t] < 0 ? adj[t].len : nx[t];
-    for (int32_t q = 0; q < k; q++)
-      if (s.cid_of[x[q].h] < c) list.push_back({s.cid_of[x[q].h], x[q].L, x[q].C});
-    std::sort(list.begin(), list.end(), [](const Ent &p, const Ent &q) { return p.h < q.h; });
-    for (const Ent &p : list) {
-      s.xtid.push_back(p.h);
-      s.eL.push_back(p.L);
-      s.eC.push_back(p.C);
+  core_ranges(n, [&](int32_t c0, int32_t c1) {
+    for (int32_t c = c0; c < c1; c++) {
+      const Ent *x = list_of(s.tid_of[c]);
+      for (int32_t q = 0; q < length_of(s.tid_of[c]); q++) s.xoff[c + 1] += s.cid_of[x[q].h] < c;
     }
-    if (s.xtid.size() >= (size_t)INT_MAX / 2) return false;
-    s.xoff[c + 1] = (int32_t)s.xtid.size();
+  });
+  int64_t total = 0;
+  for (int32_t c = 0; c < n; c++) {
+    total += s.xoff[c + 1];
+    if (total >= INT_MAX / 2) return false;
+    s.xoff[c + 1] = (int32_t)total;
   }
-  const int32_t E = (int32_t)s.xtid.size();
+  const int32_t E = (int32_t)total;
+  s.xtid.resize((size_t)E);
+  s.eL.resize((size_t)E);
+  s.eC.resize((size_t)E);
+  core_ranges(n, [&](int32_t c0, int32_t c1) {
+    for (int32_t c = c0; c < c1; c++) {
+      Ent *x = list_of(s.tid_of[c]);
+      const int32_t k = length_of(s.tid_of[c]);
+      std::sort(x, x + k, [&](const Ent &p, const Ent &q) { return s.cid_of[p.h] < s.cid_of[q.h]; });
+      for (int32_t q = 0, e = s.xoff[c]; e < s.xoff[c + 1]; q++, e++) {  // (those below c come first)
+        s.xtid[e] = s.cid_of[x[q].h];
+        s.eL[e] = x[q].L;
+        s.eC[e] = x[q].C;
+      }
+    }
+  });
   const int4 none = make_int4(-1, 0, -1, 0);
   s.arc.assign((size_t)s.nc * 4, none);
   s.info.assign((size_t)s.nc * 4, make_int4(0, 0, 0, 0));
   s.more.assign(1, none);  // (~0 would read as an absent arc)
   for (int32_t c = 0; c < s.nc; c++) {
-    const int32_t t = s.tid_of[c];
-    const Ent *x = pool.data() + adj[t].off;
-    const int32_t k = adj[t].len, direct = k > 8 ? 7 : k;
+    const int32_t k = adj[s.tid_of[c]].len;
     if (k > 60000) return false;  // (in-degrees are summed in 16 bits)
-    auto place = [&](int32_t h) {  // flow from h to c: down (c is the smaller end) or up
-      const int32_t own = std::max(h, c), other = std::min(h, c);
-      const int32_t e = (int32_t)(std::lower_bound(s.xtid.begin() + s.xoff[own], s.xtid.begin() + s.xoff[own + 1], other) - s.xtid.begin());
-      return c < h ? e : E + e;
-    };
-    for (int32_t q = 0; q < k; q++) {
-      const int32_t h = s.cid_of[x[q].h], w = place(h);
-      if (q < direct) {
-        int4 &p = s.arc[(size_t)c * 4 + q / 2], &f = s.info[(size_t)c * 4 + q / 2];
-        (q & 1 ? p.z : p.x) = h;
-        (q & 1 ? p.w : p.y) = x[q].L;
-        (q & 1 ? f.z : f.x) = x[q].C;
-        (q & 1 ? f.w : f.y) = w;
-      } else {
-        if (q == direct) s.arc[(size_t)c * 4 + 3].z = ~(int32_t)s.more.size();
-        s.more.push_back(make_int4(h, x[q].L, x[q].C, w));
-        s.arc[(size_t)c * 4 + 3].w = (int32_t)s.more.size();
+    if (k <= 8) continue;
+    s.arc[(size_t)c * 4 + 3].z = ~(int32_t)s.more.size();
+    s.more.resize(s.more.size() + k - 7);
+    s.arc[(size_t)c * 4 + 3].w = (int32_t)s.more.size();
+  }
+  core_ranges(s.nc, [&](int32_t c0, int32_t c1) {
+    for (int32_t c = c0; c < c1; c++) {
+      const int32_t t = s.tid_of[c], k = adj[t].len, direct = k > 8 ? 7 : k;
+      const Ent *x = list_of(t);
+      for (int32_t q = 0; q < k; q++) {
+        const int32_t h = s.cid_of[x[q].h], own = std::max(h, c), other = std::min(h, c);
+        const int32_t e = (int32_t)(std::lower_bound(s.xtid.begin() + s.xoff[own], s.xtid.begin() + s.xoff[own + 1], other) -
+                                    s.xtid.begin());
+        const int32_t place = c < h ? e : E + e;  // flow from h to c: down (c is the smaller end) or up
+        if (q < direct) {
+          int4 &p = s.arc[(size_t)c * 4 + q / 2], &f = s.info[(size_t)c * 4 + q / 2];
+          (q & 1 ? p.z : p.x) = h;
+          (q & 1 ? p.w : p.y) = x[q].L;
+          (q & 1 ? f.z : f.x) = x[q].C;
+          (q & 1 ? f.w : f.y) = place;
+        } else {
+          s.more[~s.arc[(size_t)c * 4 + 3].z + q - direct] = make_int4(h, x[q].L, x[q].C, place);
+        }
       }
     }
-  }
+  });
   return s.nc >= 1;
 }

@@ -37,8 +37,12 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <climits>
 #include <cstdlib>
+#include <memory>
+#include <system_error>
+#include <thread>
 #include <type_traits>
 
 #include "device_state.h"
