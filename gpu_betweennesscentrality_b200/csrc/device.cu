@@ -3634,41 +3634,33 @@ void host_rows(Handle &h, const int32_t *sources0, int32_t ns, int32_t *dist, ui
   DeviceState *d = need_dev(h);
   cudaStream_t st = d->s_label;
   const int32_t n = d->n;
-  int32_t *o_d = nullptr, *o_h = nullptr;
-  uint32_t *o_c = nullptr;
   const int32_t step = std::min<int32_t>(d->chunk, 256);
-  o_d = dmalloc<int32_t>(d, (size_t)step * n);
-  if (cnt) o_c = dmalloc<uint32_t>(d, (size_t)step * n);
-  if (hop) o_h = dmalloc<int32_t>(d, (size_t)step * n);
-  try {
-    int32_t *ds = stage_sources(d, sources0, ns, n);
-    for (int32_t off = 0; off < ns; off += step) {
-      const int32_t c = std::min(step, ns - off);
-      k_vid_to_tid<<<(c + 255) / 256, 256, 0, st>>>(ds + off, d->tid_of, d->src[0], c, n, d->err);
-      CK(cudaGetLastError());
-      launch_label(h, d, 0, d->src[0], c, false, st);
-      if (h.host.kind == IndexKind::H2H && (cnt || hop)) {
-        // sigma and waves by the Kahn pass; BC accumulation goes to a scratch target
-        CK(cudaMemsetAsync(d->bc_tid, 0, (size_t)n * 8, st));
-        launch_dep(h, d, 0, d->src[0], c, st);
-      }
-      dim3 grid((n + 255) / 256, c);
-      k_rows_to_vid<<<grid, 256, 0, st>>>(d->rec[0], d->hop[0], d->vid_of, n, d->n_pad, c, o_d, o_c, o_h);
-      CK(cudaGetLastError());
-      CK(cudaMemcpyAsync(dist + (size_t)off * n, o_d, (size_t)c * n * 4, cudaMemcpyDeviceToHost, st));
-      if (cnt) CK(cudaMemcpyAsync(cnt + (size_t)off * n, o_c, (size_t)c * n * 4, cudaMemcpyDeviceToHost, st));
-      if (hop) CK(cudaMemcpyAsync(hop + (size_t)off * n, o_h, (size_t)c * n * 4, cudaMemcpyDeviceToHost, st));
-      CK(cudaStreamSynchronize(st));
+  // The rows in vertex order take the place of the queue and layer rows, which are done with once the
+  // records and layers stand (three buffers of a call's own, 154 MB at 50k vertices, cost their
+  // cudaMalloc and cudaFree each time).
+  int32_t *o_d = d->order[0], *o_h = d->lcnt[0] + (size_t)step * n;
+  uint32_t *o_c = reinterpret_cast<uint32_t *>(d->lcnt[0]);
+  int32_t *ds = stage_sources(d, sources0, ns, n);
+  for (int32_t off = 0; off < ns; off += step) {
+    const int32_t c = std::min(step, ns - off);
+    k_vid_to_tid<<<(c + 255) / 256, 256, 0, st>>>(ds + off, d->tid_of, d->src[0], c, n, d->err);
+    CK(cudaGetLastError());
+    launch_label(h, d, 0, d->src[0], c, false, st);
+    if (h.host.kind == IndexKind::H2H && (cnt || hop)) {
+      // sigma and waves by the Kahn pass; BC accumulation goes to a scratch target
+      CK(cudaMemsetAsync(d->bc_tid, 0, (size_t)n * 8, st));
+      launch_dep(h, d, 0, d->src[0], c, st);
     }
-    check_err(d);
-  } catch (...) {
-    cudaFree(o_d); if (o_c) cudaFree(o_c); if (o_h) cudaFree(o_h);
-    throw;
+    dim3 grid((n + 255) / 256, c);
+    k_rows_to_vid<<<grid, 256, 0, st>>>(d->rec[0], d->hop[0], d->vid_of, n, d->n_pad, c, o_d, cnt ? o_c : nullptr,
+                                        hop ? o_h : nullptr);
+    CK(cudaGetLastError());
+    CK(cudaMemcpyAsync(dist + (size_t)off * n, o_d, (size_t)c * n * 4, cudaMemcpyDeviceToHost, st));
+    if (cnt) CK(cudaMemcpyAsync(cnt + (size_t)off * n, o_c, (size_t)c * n * 4, cudaMemcpyDeviceToHost, st));
+    if (hop) CK(cudaMemcpyAsync(hop + (size_t)off * n, o_h, (size_t)c * n * 4, cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
   }
-  cudaFree(o_d);
-  if (o_c) cudaFree(o_c);
-  if (o_h) cudaFree(o_h);
-  d->bytes -= (int64_t)step * n * 4 * (1 + (cnt ? 1 : 0) + (hop ? 1 : 0));
+  check_err(d);
 }
 
 // ------------------------------------------------------------------ allocation-free single source
