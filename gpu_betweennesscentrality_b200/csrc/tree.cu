@@ -101,6 +101,11 @@ struct TreeArgs {
 
 __device__ __forceinline__ bool wrapped(const TreeArgs &a) { return __ldcg(a.wrap) != 0; }
 
+// Launched by launch_early, a kernel starts while the one before it still runs: what it reads above
+// wait_before must be older than that one, and lets the next one start from let_next on.
+__device__ __forceinline__ void let_next() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void wait_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 __device__ __forceinline__ uint32_t count_of(const TreeArgs &a, unsigned long long c) {
   if (c > 0x7fffffffull) {
     *a.wrap = 1;
@@ -898,7 +903,7 @@ __device__ __forceinline__ void load_table(const TreeArgs &a, int start, int len
 __global__ void __launch_bounds__(kPieceLen * 32) k_trunk_down_narrow(TreeArgs a, int piece0) {
   __shared__ PieceTable p;
   __shared__ uint2 row_d[2][32], row_c[2][32];
-  if (__syncthreads_or(wrapped(a))) return;
+  let_next();
   const int4 pc = a.piece[piece0 + blockIdx.x];
   const int start = pc.x, len = pc.y - pc.x, g = blockIdx.y;
   const int i = threadIdx.x >> 5, lane = threadIdx.x & 31;  // this warp's vertex
@@ -907,12 +912,14 @@ __global__ void __launch_bounds__(kPieceLen * 32) k_trunk_down_narrow(TreeArgs a
   load_table(a, start, len, p);
   unsigned md[2] = {}, ar[2] = {}, hits[2] = {}, over = 0;
   uint32_t cnt[2] = {};
+  int s[2];
+  bool live[2];
+  lane_sources(a, g, lane, s, live);
+  const int4 m = a.tmeta[start + min(i, len - 1)];
+  const int2 sub = a.tsub[start + min(i, len - 1)];
+  wait_before();
+  if (__syncthreads_or(wrapped(a))) return;
   if (i < len) {
-    int s[2];
-    bool live[2];
-    lane_sources(a, g, lane, s, live);
-    const int4 m = a.tmeta[start + i];
-    const int2 sub = a.tsub[start + i];
     const size_t u = ((size_t)g * a.H + sub.y) * kGroup + 2 * lane;
     unsigned m1[2], m2[2];
 #pragma unroll
@@ -975,7 +982,7 @@ __global__ void __launch_bounds__(kPieceLen * 32) k_trunk_up_narrow(TreeArgs a, 
   __shared__ PieceTable p;
   __shared__ double2 row_f[2][32];
   __shared__ uint2 row_a[2][32], row_s[2][32], row_d[2][32];
-  if (__syncthreads_or(wrapped(a))) return;
+  let_next();
   const int4 pc = a.piece[piece0 + blockIdx.x];
   const int start = pc.x, len = pc.y - pc.x, g = blockIdx.y;
   const int i = threadIdx.x >> 5, lane = threadIdx.x & 31;  // this warp's vertex
@@ -989,8 +996,7 @@ __global__ void __launch_bounds__(kPieceLen * 32) k_trunk_up_narrow(TreeArgs a, 
   unsigned ar[2] = {};
   uint2 st = make_uint2(0, 0), dt = st;
   lane_sources(a, g, lane, s, live);
-  if (i < len) {
-    const double2 j = __ldcg(reinterpret_cast<const double2 *>(a.J + own));
+  if (i < len) {  // (all but the flow is the way down's)
     const uint2 x = *reinterpret_cast<const uint2 *>(a.arg + own);
     st = *reinterpret_cast<const uint2 *>(a.S + own);
     dt = *reinterpret_cast<const uint2 *>(a.D + own);
@@ -1000,7 +1006,6 @@ __global__ void __launch_bounds__(kPieceLen * 32) k_trunk_up_narrow(TreeArgs a, 
       si[k] = a.tidx_of[s[k]];
       if (!live[k]) continue;  // a lane without a source has no flow and no argument
       ar[k] = k ? x.y : x.x;
-      f[k] = (k ? j.y : j.x) + (m.w != s[k] ? 1.0 : 0.0);
     }
 #pragma unroll
     for (int k = 0; k < 2; k++) {
@@ -1009,6 +1014,14 @@ __global__ void __launch_bounds__(kPieceLen * 32) k_trunk_up_narrow(TreeArgs a, 
     }
   }
   load_table(a, start, len, p);
+  wait_before();
+  if (__syncthreads_or(wrapped(a))) return;
+  if (i < len) {
+    const double2 j = __ldcg(reinterpret_cast<const double2 *>(a.J + own));
+#pragma unroll
+    for (int k = 0; k < 2; k++)
+      if (live[k]) f[k] = (k ? j.y : j.x) + (m.w != s[k] ? 1.0 : 0.0);
+  }
   for (int t = len - 1; t > 0; t--) {
     if (t == i) {
       row_f[t & 1][lane] = make_double2(f[0], f[1]);
@@ -1522,8 +1535,9 @@ __device__ __forceinline__ void unpack_one(const int4 t, const int32_t *eC, doub
 }
 
 // A level of triangles is final once the levels before it are done: a launch per large level, and
-// the small ones at the end (a few thousand triangles each) by one CTA with barriers between them
-// instead of a launch each.
+// the small ones at the end by one cluster, a triangle per thread, with cluster barriers between them.
+// A level is a chain of latencies (its B, the atomics, the barrier), so the next level's triangle and
+// share, which no level changes, are loaded before the barrier.
 __global__ void k_unpack(const int4 *__restrict__ tri, int64_t count, const int32_t *__restrict__ eC, double *B, double *F,
                          const int32_t *wrap) {
   if (__ldcg(wrap) != 0) return;
@@ -1531,16 +1545,38 @@ __global__ void k_unpack(const int4 *__restrict__ tri, int64_t count, const int3
   if (k < count) unpack_one(tri[k], eC, B, F);
 }
 
-constexpr int64_t kTailLevel = 8192;  // triangles of a level that the one-CTA form takes
-__global__ void __launch_bounds__(1024) k_unpack_tail(const int4 *__restrict__ tri, const int64_t *__restrict__ at, int l0,
-                                                      int l1, const int32_t *__restrict__ eC, double *B, double *F,
-                                                      const int32_t *wrap) {
-  if (__ldcg(wrap) != 0) return;  // (not written while this kernel runs)
+constexpr int kTailCtas = 8;
+constexpr int64_t kTailLevel = kTailCtas * 1024;  // triangles of a level that the cluster takes
+__global__ void __cluster_dims__(kTailCtas, 1, 1) __launch_bounds__(1024)
+    k_unpack_tail(const int4 *__restrict__ tri, const int64_t *__restrict__ at, int l0, int l1, const int32_t *__restrict__ eC,
+                  double *B, double *F, const int32_t *wrap) {
+  if (__ldcg(wrap) != 0) return;  // (not written while this kernel runs, so the same for all)
+  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  int4 t = make_int4(0, 0, 0, 0);
+  double part = 0.0;  // 0: no triangle
+  auto load = [&](int l) {
+    const int64_t b = at[l], e = at[l + 1];
+    part = 0.0;
+    if (b + k >= e) return;
+    t = tri[b + k];
+    const int c1 = eC[t.x], c3 = eC[t.z];
+    part = c3 == 1 ? 1.0 : share(c1, (uint32_t)eC[t.y], (uint32_t)c3);
+  };
+  load(l0);
   for (int l = l0; l < l1; l++) {
-    const int64_t e = at[l + 1];
-    for (int64_t k = at[l] + threadIdx.x; k < e; k += blockDim.x) unpack_one(tri[k], eC, B, F);
+    if (part != 0.0) {
+      const double w = __ldcg(B + t.z) * part;
+      if (w != 0.0) {
+        atomicAdd(B + t.x, w);
+        atomicAdd(B + t.y, w);
+        atomicAdd(F + t.w, w);
+      }
+    }
+    if (l + 1 == l1) break;
+    load(l + 1);
     __threadfence();
-    __syncthreads();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   }
 }
 
@@ -2278,6 +2314,21 @@ static void launch_bottom(const TreeArgs &a, int first, int end, int rows, cudaS
   k_bottom<<<dim3(end - first, (a.ng + gpc - 1) / gpc), warps * 32, smem, st>>>(a, first, rows, gpc);
 }
 
+// The kernel may, if early, start before the one ahead of it in the stream ends (see wait_before).
+template <class... A, class... B>
+static void launch_early(void (*kernel)(A...), bool early, dim3 grid, int threads, cudaStream_t st, B... args) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = grid;
+  c.blockDim = dim3((unsigned)threads);
+  c.stream = st;
+  c.attrs = &at;
+  c.numAttrs = early ? 1 : 0;
+  CK(cudaLaunchKernelEx(&c, kernel, static_cast<A>(args)...));
+}
+
 static void launch_bottoms(DeviceState *d, const TreeArgs &a, cudaStream_t st) {
   const TreePlan &p = *d->tree;
   if (a.ng > 4) {
@@ -2312,7 +2363,7 @@ static void launch_unpack(DeviceState *d, cudaStream_t st) {
     launched();
   }
   if (p.tail_level < top) {
-    k_unpack_tail<<<1, 1024, 0, st>>>(p.tri, p.tri_at, p.tail_level, top, a.eC, a.Bd, a.F, a.wrap);
+    k_unpack_tail<<<kTailCtas, 1024, 0, st>>>(p.tri, p.tri_at, p.tail_level, top, a.eC, a.Bd, a.F, a.wrap);
     launched();
   }
 }
@@ -2458,7 +2509,7 @@ void launch_tree(const Handle &h, DeviceState *d, const int32_t *d_src_tid, int3
     for (int l = 0; l < levels; l++) {
       const int32_t *c = p.level_class.data() + 4 * l;
       if ((int64_t)(c[3] - c[0]) * a.ng < kWideCtas) {
-        k_trunk_down_narrow<<<dim3(c[3] - c[0], a.ng), kPieceLen * 32, 0, st>>>(a, c[0]);
+        launch_early(k_trunk_down_narrow, l > 0, dim3(c[3] - c[0], a.ng), kPieceLen * 32, st, a, c[0]);
         launched();
         continue;
       }
@@ -2484,7 +2535,7 @@ void launch_tree(const Handle &h, DeviceState *d, const int32_t *d_src_tid, int3
     for (int l = levels - 1; l >= 0; l--) {
       const int32_t *c = p.level_class.data() + 4 * l;
       if ((int64_t)(c[3] - c[0]) * a.ng < kWideCtas) {
-        k_trunk_up_narrow<<<dim3(c[3] - c[0], a.ng), kPieceLen * 32, 0, st>>>(a, c[0]);
+        launch_early(k_trunk_up_narrow, l < levels - 1, dim3(c[3] - c[0], a.ng), kPieceLen * 32, st, a, c[0]);
         launched();
         continue;
       }
