@@ -34,6 +34,9 @@
 // Counts are held in 32 bits as in the label rows.  Those wrap where the true count passes 2^31, and
 // BC is then defined by the wrapped values; here a product that reaches 2^31 sets the wrap word, the
 // kernels leave their results unused, and the call is answered by the label kernels.
+//
+// All 50,175 sources of the 50k grid: 239.8 ms by the label kernels (label scan 142, dependency pass
+// 77, sorting and gaps), 38.3 ms so; 1,024 sources of 500k 150.8 and 22.1 ms, 6,083 of 6k 3.31 and 1.20.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -57,6 +60,7 @@ constexpr unsigned kNoKey = 0xffffffffu;
 constexpr int kGroup = 64;           // sources a warp takes: two neighbouring ones per lane
 constexpr int kPieceLen = 32;        // trunk vertices per piece
 // a bottom subtree: rows in shared memory (its separator and its vertices with descendants), vertices, edges
+// (12, 16, 20 rows, all sources of 50k: 43.3, 42.5, 43.2 ms)
 constexpr int kBottomRows = 16;
 constexpr int kBottomVerts = 64;
 constexpr int kBottomEdges = 224;
@@ -881,7 +885,9 @@ __global__ void __launch_bounds__(Wide<PL>::warps * 32) k_trunk_up(TreeArgs a, i
 // vertex.  The path is followed vertex by vertex: a vertex's warp publishes its distances and counts,
 // and the warps of the vertices below offer them to their running minimum, arguments and count in
 // registers.  (One warp walking the path alone takes 23k cycles for the distances and 16k for the
-// counts of a full piece.)
+// counts of a full piece.)  256 sources of 50k vertices are 18 levels of 28 us each way, bound by that
+// chain (issue 5 %, DRAM below 1 %); 16 or 32 distances of a scan in flight instead of 8 changed nothing
+// (1.29, 1.33 and 1.30 ms).  A level starts while the one before it runs (let_next): 1.41 -> 1.34 ms.
 struct PieceTable {
   unsigned win[kPieceLen][kPieceLen + 1];  // key of the edge (vertex, earlier vertex), or absent
   int cin[kPieceLen][kPieceLen + 1];       // its count
@@ -1063,7 +1069,8 @@ __global__ void __launch_bounds__(kPieceLen * 32) k_trunk_up_narrow(TreeArgs a, 
 // per vertex and warp): that entry's flow stays in the finished row and is summed after the pass,
 // eight rows at a time, instead of by a warp-wide sum per vertex.
 //
-// The pass is bound by instruction issue and by the warps that shared memory leaves room for, so
+// The pass is bound by instruction issue and by the warps that shared memory leaves room for (50k: issue
+// 32 to 38 % with 9 to 15 warps per SM, DRAM 5 to 11 %; a third of the time of all sources), so
 // shared memory is addressed by 32-bit offsets (ld.shared / st.shared); a row's block holds delta
 // (f64), distance, count and argument of the warp's sources.
 constexpr int kTieCode = 0xff, kSkipCode = 0xfe;  // arguments that are no row: a tie, a lane without a source
@@ -1537,7 +1544,8 @@ __device__ __forceinline__ void unpack_one(const int4 t, const int32_t *eC, doub
 // A level of triangles is final once the levels before it are done: a launch per large level, and
 // the small ones at the end by one cluster, a triangle per thread, with cluster barriers between them.
 // A level is a chain of latencies (its B, the atomics, the barrier), so the next level's triangle and
-// share, which no level changes, are loaded before the barrier.
+// share, which no level changes, are loaded before the barrier: 55 us for the last levels at 50k
+// vertices, 94 with one CTA and up to eight triangles per thread.
 __global__ void k_unpack(const int4 *__restrict__ tri, int64_t count, const int32_t *__restrict__ eC, double *B, double *F,
                          const int32_t *wrap) {
   if (__ldcg(wrap) != 0) return;
@@ -2249,10 +2257,14 @@ static size_t group_bytes(const TreePlan &p) {
   return ((size_t)a.NT * (4 + 4 + 4 + 8) + (size_t)a.H * (4 + 4 + 8)) * kGroup;
 }
 
-constexpr int64_t kWideCtas = 148 * 12;  // (piece, group) pairs from which a level is wide
+// (piece, group) pairs from which a level is wide: below, the narrow kernels' shorter chain per piece
+// counts, above, how many pieces an SM has in flight.  2, 12, 32 and 48 per SM: 1.69, 1.41, 1.43,
+// 1.43 ms (50k vertices, 256 sources), 49.3, 49.5, 50.3, 56.6 ms (50k, all; an earlier state), 1.33,
+// 1.36, 1.44, 1.73 ms (6k, all).
+constexpr int64_t kWideCtas = 148 * 12;
 
 // Groups of sources that the per-source scratch holds, at most kMaxGroups.
-constexpr int kMaxGroups = 1024;
+constexpr int kMaxGroups = 1024;  // (all sources of 50k in passes of 96, 192, 264 groups: 44.3, 39.1, 37.2 ms)
 static int groups_fit(const DeviceState *d) {
   const size_t room = (size_t)d->chunk * d->n_pad * sizeof(int4);
   size_t fit = std::min<size_t>(kMaxGroups, room / group_bytes(*d->tree));
@@ -2303,14 +2315,21 @@ bool tree_disable(DeviceState *d) {
   return true;
 }
 
+// The attribute belongs to the function, not to a launch, and other threads launch it for other
+// indexes: every launch sets the same limit, the one that the plans are checked against.
+template <class K>
+static void allow_smem(K kernel, size_t bytes) {
+  CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+}
+
 // The bottoms [first, end) of at most `rows` rows: the warps of a CTA share a bottom's edges, and a
 // CTA takes more groups one after another while there are CTAs enough.
 static void launch_bottom(const TreeArgs &a, int first, int end, int rows, cudaStream_t st) {
   const int warps = std::min(kBottomWarps, a.ng);
   int gpc = warps;
   while (gpc < 64 && (int64_t)(end - first) * ((a.ng + 2 * gpc - 1) / (2 * gpc)) >= 148 * 24) gpc *= 2;
+  static_assert(kBottomWarps * kBottomRows * RowLayout::size <= 36 * 1024, "no opt-in for more than 48 KB");
   const size_t smem = (size_t)warps * rows * RowLayout::size;
-  CK(cudaFuncSetAttribute(k_bottom, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   k_bottom<<<dim3(end - first, (a.ng + gpc - 1) / gpc), warps * 32, smem, st>>>(a, first, rows, gpc);
 }
 
@@ -2428,7 +2447,7 @@ static void launch_core(const Handle &h, DeviceState *d, const int32_t *d_src_ti
     const int threads = core_threads(h, a.ns, nc);
     const CoreKernels kernels = core_kernels(threads);
     const size_t smem = (size_t)core_words(nc) * 8;
-    CK(cudaFuncSetAttribute(kernels.sweep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_smem(kernels.sweep, (size_t)d->smem_optin - 8192);
     if (d->profiling) {
       ev = take_events(d->ev_lab, d->ev_lab_used);
       CK(cudaEventRecord(ev.first, st));
@@ -2502,7 +2521,7 @@ void launch_tree(const Handle &h, DeviceState *d, const int32_t *d_src_tid, int3
       launched();
     } else {
       const size_t smem = (size_t)p.up_warps * a.H * 8;
-      CK(cudaFuncSetAttribute(k_up_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      allow_smem(k_up_rows, (size_t)d->smem_optin - 2048);
       k_up_rows<<<(a.ng * kGroup + p.up_warps - 1) / p.up_warps, p.up_warps * 32, smem, st>>>(a);
       launched();
     }
@@ -2555,7 +2574,7 @@ void launch_tree(const Handle &h, DeviceState *d, const int32_t *d_src_tid, int3
     {
       const size_t smem = (size_t)a.H * 20;
       auto kern = a.ns >= 148 * 8 ? k_up_back<4> : k_up_back<8>;
-      CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      allow_smem(kern, (size_t)d->smem_optin - 2048 - sizeof(BackShared<8>));
       kern<<<a.ns, a.ns >= 148 * 8 ? 128 : 256, smem, st>>>(a);
       launched();
     }
