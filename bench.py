@@ -3,8 +3,9 @@ other configurations of the workload as extra keys.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl b200|reference] [--n 50000]
 
-One step = one full pass of the hot path over the workload: BC from all n sources (n source
-sweeps: label scan for dist/count/hop rows, SP-DAG level bucketing, FP64 dependency backprop).
+One step = one full pass of the hot path over the workload: BC from all n sources (distances and path
+counts of every pair down the elimination tree, FP64 dependencies up it, the flow through shortcuts
+unpacked; with a tuning that asks for a label kernel: label scan, SP-DAG level bucketing, backprop).
 `value` is whole-job sources/s timed with CUDA events on the launching stream (index resident in
 HBM); `e2e` is the same metric through the public C-ABI call with host buffers (source list H2D,
 BC D2H inside the timed region).  With N>1 ranks (torchrun) each rank sweeps a contiguous share
@@ -275,8 +276,33 @@ def plain_rate(idx, sources, k):
 L2_BYTES = 126e6
 
 
+LABEL_FIELDS = ("lanes_per_source", "split", "dep_form", "queue_depth", "label_warps", "label_tile", "label_passes",
+                "label_sources", "label_stream")
+
+
+def tree_roofline(idx, shard, n, stats, steps, peak, peak_src):
+    """BC over the elimination tree (tree.cu).  What a step has to read is small: the sources' label
+    rows (12 B per entry) and the BC vector; the rows of the trunk are written and read in L2-sized
+    passes.  So the HBM fraction is near zero by design; the kernels are bound by instruction issue
+    and by latency at the occupancy that their shared-memory rows leave (profiles/tree_sweep_50k.md).
+    down: U rows, trunk levels, bottoms (down and up); up: trunk levels in reverse, U rows in reverse;
+    what is left of the step is the unpacking."""
+    entries = idx.info()[7] * len(shard) / n
+    need = 12.0 * entries + 8.0 * n
+    down, up = stats["label_ms"] / steps, stats["dep_ms"] / steps
+    achieved = need / ((down + up) / 1e3) / 1e9
+    return {"bound": "issue and latency", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
+            "traffic": None, "peak_source": peak_src, "kernel": "k_bottom, k_trunk_down, k_trunk_up",
+            "needed_bytes_per_step": need, "passes_per_step": stats["label_launches"] / steps,
+            "launches_per_step": stats["launches"] / steps, "down_ms_per_step": down, "up_ms_per_step": up,
+            "pairs_per_s": len(shard) * float(n) / ((down + up) / 1e3),
+            "note": "frac = bytes a step has to read and write / time of its sweeps / measured HBM copy bandwidth: "
+                    "the sweep keeps its rows on the chip, so this is small by design; issue, occupancy and DRAM "
+                    "counters of the kernels are in profiles/"}
+
+
 def label_roofline(idx, shard, n, stats, steps, peak, peak_src, sm_mhz):
-    """Dominant kernel of the label path: the packed label scan.  DRAM model per launch: the target
+    """The label kernels, where the tuning asks for one; else the tree's.  Dominant kernel of the label path: the packed label scan.  DRAM model per launch: the target
     rows' label distances -- read once per launch when the distance array fits in three quarters
     of the L2 (50k: 69 MB; every CTA group then finds them in L2), else once per CTA group of sources (32;
     16 for the lane-pair forms), each row up to the group's deepest LCA depth (4 B per entry, exact
@@ -286,6 +312,8 @@ def label_roofline(idx, shard, n, stats, steps, peak, peak_src, sm_mhz):
     algorithmic figure of the workload's byte model (12 B per label entry scanned + 12 B per pair)
     is given as effective_bw: rows are reused by every source of a group, so it exceeds the HBM
     peak."""
+    if not any(idx.get_tuning().get(k) for k in LABEL_FIELDS):
+        return tree_roofline(idx, shard, n, stats, steps, peak, peak_src)
     ns = len(shard)
     per_cta = idx.label_group() or 32
     tall = per_cta == 16
@@ -326,23 +354,22 @@ def label_roofline(idx, shard, n, stats, steps, peak, peak_src, sm_mhz):
 
 
 def sweep_roofline(n, ns_step, stats, steps, peak, peak_src):
-    """The label-free sweep kernel (k_sweep_rows).  DRAM model per source: each 16-byte record is
-    initialised (16 B), then read and rewritten by the in-degree pass (32 B) -- 48 B per vertex (the
-    batched sweep writes no hop layers: the dependency pass reads its wave queue); the frontier
-    phases' scattered record visits come on top (DRAM sectors per visit), which ncu's traffic in
-    profiles/ shows (~415 B per (source, vertex) at 200k + 2 %)."""
+    """The label-free index's sweep over the core graph (core.cuh).  DRAM model per source: a core
+    vertex (30 % of the vertices on these graphs) has 28 B of state and rows (distance 4, count word 8,
+    rows of distances, counts and dependencies 16), written and read once; the frontier's scattered
+    visits come on top where they miss L2.  sweep: U rows, core sweep, rows, bottoms; dependency: core
+    waves in reverse and the way back."""
     ms_step = stats["label_ms"] / steps
+    dep_step = stats["dep_ms"] / steps
     launches_step = max(1.0, stats["label_launches"] / steps)
-    launch_ms = ms_step / launches_step
-    dram_step = 48.0 * n * ns_step
-    achieved = dram_step / launches_step / (launch_ms / 1e3) / 1e9
-    return {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-            "traffic": None, "peak_source": peak_src, "kernel": "k_sweep_rows",
-            "dram_model_bytes_per_launch": dram_step / launches_step, "launch_ms": launch_ms,
-            "launches_per_step": launches_step, "sweep_ms_per_step": ms_step,
-            "dependency_ms_per_step": stats["dep_ms"] / steps,
-            "note": "model = 48 B per (source, vertex): record init, in-degree pass read + write; the scattered "
-                    "frontier visits are gathers of DRAM sectors (ncu: ~415 B per (source, vertex) moved)"}
+    dram_step = 56.0 * 0.3 * n * ns_step
+    achieved = dram_step / ((ms_step + dep_step) / 1e3) / 1e9
+    return {"bound": "latency", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
+            "traffic": None, "peak_source": peak_src, "kernel": "k_core_sweep, k_core_dep, k_bottom",
+            "dram_model_bytes_per_pass": dram_step / launches_step, "passes_per_step": launches_step,
+            "sweep_ms_per_step": ms_step, "dependency_ms_per_step": dep_step,
+            "note": "model = 17 B per (source, vertex): 28 B of a core vertex written and read once; the sweep "
+                    "waits for scattered loads (ncu figures of the kernels are in profiles/)"}
 
 
 # ------------------------------------------------------------------------------- RQ (batched / served)
@@ -422,7 +449,7 @@ def config_shortcuts_1m(q, args, dev, flush, peak, peak_src):
     e2e, _ = e2e_rate(idx, sample, 2)
     plain, k_plain = plain_rate(idx, sample, 8)
     out = {"workload": f"batched / served RQ on the seeded {n}-vertex perturbed grid + 2% random shortcut edges "
-                       f"(weights 500..5000), label-free index (per-source shortest-path sweeps); a seeded sample of "
+                       f"(weights 500..5000), label-free index (per-source shortest-path sweeps over the core graph); a seeded sample of "
                        f"{len(sample)} sources per step (partial BC)",
            "n": n, "arcs": int(idx.info()[1]), "sources_per_step": int(len(sample)), "steps": steps, "warmup": 3,
            "value": value, "unit": "sources/s", "ms_per_step": sum(ms) / steps,
@@ -443,9 +470,9 @@ def config_shortcuts_1m(q, args, dev, flush, peak, peak_src):
 
 
 def config_mhl_1m(q, args, dev, flush, peak, peak_src):
-    """The label path on a tree too tall for the 32-source label kernel: MHL-QBC partial BC on the
+    """The label index of a tall tree: MHL-QBC partial BC on the
     1,000,000-vertex grid without shortcuts (tree height 2,725), rows filled on the device (its
-    last 16,384 eliminations too), default tuning: the 16-source tall-tree label kernel."""
+    last 16,384 eliminations too), default tuning: BC over the elimination tree."""
     import torch
     from gpu_betweennesscentrality_b200 import synth
 
@@ -470,7 +497,7 @@ def config_mhl_1m(q, args, dev, flush, peak, peak_src):
     e2e, _ = e2e_rate(idx, sample, 1)
     roof = label_roofline(idx, sample, n, stats, steps, peak, peak_src, clk.get("sm_mhz") or 1965.0)
     out = {"workload": f"MHL-QBC partial BC over a seeded sample of {len(sample)} sources, seeded perturbed grid "
-                       f"n={n} without shortcuts (tree height {int(info[3])}: the tall-tree label kernel)",
+                       f"n={n} without shortcuts (tree height {int(info[3])})",
            "n": n, "sources_per_step": int(len(sample)), "steps": steps, "warmup": 3,
            "value": value, "unit": "sources/s", "ms_per_step": sum(ms) / steps,
            "e2e": {"value": e2e, "unit": "sources/s", "h2d_bytes_per_step": int(4 * len(sample)),

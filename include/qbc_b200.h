@@ -143,14 +143,20 @@ int qbc_index_export(const qbc_index *idx, int32_t *vid_of, int32_t *depth, int3
  * height fits; 0 = auto: 16 when the 32-source kernel cannot hold whole rows and [7]-[9] are 0),
  * [13]=target rows of the 16-source kernel (1 = whole rows, double-buffered per warp side; 2 =
  * 64-entry blocks through a ring; 0 = auto: whole rows when they fit with 16 warps).  Refused
- * with QBC_EBUSY while the index serves. */
+ * with QBC_EBUSY while the index serves.
+ * With [0], [2], [5]-[9], [12] and [13] all 0, BC of many (source, vertex) pairs runs over the
+ * elimination tree (label indexes built here, not loaded from a file) or over the core graph (CSR
+ * index; [10] and [11] apply, [11] = 0 chooses by the core's size) instead of the label, sweep and
+ * dependency kernels; any of those fields set asks for the latter.  A path count past 2^31 does, too,
+ * from the call that meets it on. */
 int qbc_index_set_tuning(qbc_index *idx, const int32_t *params, int32_t nparams);
 int qbc_index_get_tuning(const qbc_index *idx, int32_t *params, int32_t nparams);
 
 /* Kernel timing: after qbc_index_profile(idx, 1) every label-scan and dependency launch is
  * bracketed by CUDA events on its own stream; qbc_index_stats synchronises and returns
  * out[0]=label-scan ms, [1]=label-scan launches, [2]=dependency ms, [3]=dependency launches,
- * [4]=all kernel launches of the library since the profile call. */
+ * [4]=all kernel launches of the library since the profile call.  Over the tree or the core, [0] and
+ * [1] are the passes' way down (with the bottoms) and [2], [3] their way up. */
 int qbc_index_profile(qbc_index *idx, int on);
 int qbc_index_stats(qbc_index *idx, double *out);
 
@@ -158,13 +164,15 @@ int qbc_index_stats(qbc_index *idx, double *out);
  * threads of the label kernel, target split, dependency form and level-queue depth, chunk size --
  * on a sweep over the listed sources, keeps the fastest on the index and returns it in params
  * (layout of qbc_index_set_tuning, up to 12) with its time per source in ms.  On a CSR index
- * it tunes the sweep's bucket width and threads, the dependency threads and the chunk size. */
+ * it tunes the sweep's bucket width and threads, the dependency threads and the chunk size.  Tune on a
+ * list as long as those to come: a short one is answered by the label kernels, and the fields that it
+ * then sets keep them. */
 int qbc_autotune(qbc_index *idx, const int32_t *sources0, int32_t ns, int32_t *params, int32_t nparams,
                  double *ms_per_source);
 
 /* ---- BC (replaces Graph::brandesBCIndexGPU_5, MHLQBC.cu:495-537 / QBC.cu:419-584) ------------
- * Batched path: many sources per launch, label rows staged in shared memory, level-bucketed
- * backprop.  qbc_bc_all's sweep is captured once into a CUDA graph per tuning and replayed.
+ * Batched path: many sources per launch, over the elimination tree or a core graph, or by label
+ * rows staged in shared memory and a level-bucketed backprop (see qbc_index_set_tuning).  qbc_bc_all's sweep is captured once into a CUDA graph per tuning and replayed.
  * bc_out: n host doubles (overwritten). */
 int qbc_bc_all(qbc_index *idx, double *bc_out);
 /* partial BC over a source list (0-based vids) */
