@@ -2424,7 +2424,7 @@ void launch_chunk(const Handle &h, DeviceState *d, const int32_t *d_src_tid, int
 
 void launch_sources(const Handle &h, DeviceState *d, const int32_t *d_src_tid, int32_t ns, cudaStream_t st, bool rerun) {
   const int32_t *guard = nullptr;
-  if (use_tree(h, d, ns)) {
+  if (use_tree(h, d, ns, rerun)) {
     launch_tree(h, d, d_src_tid, ns, st);
     if (rerun) return;
     guard = tree_guard(d);

@@ -2273,19 +2273,25 @@ static int groups_fit(const DeviceState *d) {
   return (int)fit;
 }
 
-// (source, vertex) pairs from which the tree is the faster path: its launches follow the trunk level by
-// level, 0.8 to 1.1 ms at 50k vertices however few the sources, where the label kernels answer 1, 16,
-// 32, 64 sources in 0.52, 0.93, 1.02, 1.22 ms; at 6k vertices 128 sources take them 0.23 and the tree
-// 0.39 ms, 6,083 sources 3.15 and 1.20 ms.  An H2H index's label path counts paths by Kahn waves (2,024
-// sources of 2,024 vertices 1.40 and 0.47 ms).  QBC_TREE_MIN_PAIRS overrides it for tests.
-static int64_t min_pairs(const Handle &h) {
+// (source, vertex) pairs from which the tree is the faster path.  Its launches follow the trunk level by
+// level, however few the sources: 0.24, 0.31, 0.47, 0.78, 1.5 and 5.1 ms for one source of 2k, 6k, 21k,
+// 50k, 120k and 500k vertices.  The label kernels of an MHL index start lower on small graphs and rise
+// with the pairs: 0.15, 0.18, 0.33, 0.63, 1.5, 5.2 ms for one source, and the two meet at about 3.3M
+// pairs (6k: 0.492 against 0.457 ms at 3.1M), 2.2M (12k), 1.5M (21k) and 0.2M (50k: 0.820 against
+// 0.839 ms at 4 sources); a line through those.  Calls that only enqueue are followed by the guarded
+// label launches and often overlap with others, where the tree's chain has little to offer: 2M for
+// those.  An H2H index counts paths by Kahn waves on the label path, which is slower from the first
+// source on (1,023 vertices 0.196 against 0.244 ms, 21k 0.59 against 1.47).  QBC_TREE_MIN_PAIRS overrides
+// it for tests.
+static int64_t min_pairs(const Handle &h, bool rerun) {
   const char *e = std::getenv("QBC_TREE_MIN_PAIRS");
   if (e && *e) return std::strtoll(e, nullptr, 10);
   if (h.host.kind == IndexKind::CSR) return 0;  // (one source of 100 vertices 0.146 against 0.170 ms)
-  return h.host.kind == IndexKind::H2H ? (int64_t)1 << 20 : (int64_t)2 << 20;
+  if (h.host.kind == IndexKind::H2H) return rerun ? 1000 : 1 << 20;
+  return rerun ? std::max<int64_t>(0, 3600000 - 68 * (int64_t)h.host.n) : 2 << 20;
 }
 
-bool use_tree(const Handle &h, const DeviceState *d, int32_t ns) {
+bool use_tree(const Handle &h, const DeviceState *d, int32_t ns, bool rerun) {
   const Tuning &t = h.tuning;
   if (!d->tree || d->tree->off || ns < 1) return false;
   // a tuning that picks a label or dependency kernel, or the test hook of the label rows' copies, gets it
@@ -2294,7 +2300,7 @@ bool use_tree(const Handle &h, const DeviceState *d, int32_t ns) {
     return false;
   const char *hook = std::getenv("QBC_TEST_ROW_WAIT_SPINS");
   if (hook && *hook) return false;
-  return (int64_t)ns * d->n >= min_pairs(h) && groups_fit(d) >= 1;
+  return (int64_t)ns * d->n >= min_pairs(h, rerun) && groups_fit(d) >= 1;
 }
 
 bool tree_source_rows(const DeviceState *d, const int32_t *src, int32_t ns, int32_t stride, int32_t *rows, cudaStream_t st) {
