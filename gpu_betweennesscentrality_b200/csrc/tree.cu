@@ -1134,7 +1134,13 @@ __global__ void __launch_bounds__(kBottomWarps * 32) k_bottom(TreeArgs a, int fi
   __shared__ uint8_t emap[kBottomVerts][kBottomRows];  // edge of (vertex, x row)
   __shared__ uint8_t vertex_of[kBottomRows];           // of a row (less b)
   __shared__ uint8_t leaf_units[kBottomWarps][kBottomEdges];  // groups (at most 64) whose leaf handed everything to the edge
-  if (__syncthreads_or(wrapped(a))) return;
+  // Launches of one pass (a few classes of rows) read nothing that another of them writes, so they run
+  // into each other; block 0 ends after the launch before, and so do the kernels that follow.
+  let_next();
+  auto end = [] {
+    if (blockIdx.x == 0 && blockIdx.y == 0) wait_before();
+  };
+  if (__syncthreads_or(wrapped(a))) return end();
   const int4 bt = a.bot[first + blockIdx.x];
   const int r = bt.x, m = bt.y, b = bt.z, nr = bt.w - bt.z;  // nr: vertices with descendants
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
@@ -1513,6 +1519,7 @@ __global__ void __launch_bounds__(kBottomWarps * 32) k_bottom(TreeArgs a, int fi
   const int ne = a.xoff[r + m] - ebase;
   for (int i = lane; i < ne; i += 32)
     if (leaf_units[warp][i]) atomicAdd(a.Bd + ebase + i, (double)leaf_units[warp][i] * kGroup);
+  end();
 }
 
 // ------------------------------------------------------------------------------- unpack, finish
@@ -2328,42 +2335,48 @@ static void allow_smem(K kernel, size_t bytes) {
   CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
 }
 
-// The bottoms [first, end) of at most `rows` rows: the warps of a CTA share a bottom's edges, and a
-// CTA takes more groups one after another while there are CTAs enough.
-static void launch_bottom(const TreeArgs &a, int first, int end, int rows, cudaStream_t st) {
-  const int warps = std::min(kBottomWarps, a.ng);
-  int gpc = warps;
-  while (gpc < 64 && (int64_t)(end - first) * ((a.ng + 2 * gpc - 1) / (2 * gpc)) >= 148 * 24) gpc *= 2;
-  static_assert(kBottomWarps * kBottomRows * RowLayout::size <= 36 * 1024, "no opt-in for more than 48 KB");
-  const size_t smem = (size_t)warps * rows * RowLayout::size;
-  k_bottom<<<dim3(end - first, (a.ng + gpc - 1) / gpc), warps * 32, smem, st>>>(a, first, rows, gpc);
-}
-
 // The kernel may, if early, start before the one ahead of it in the stream ends (see wait_before).
 template <class... A, class... B>
-static void launch_early(void (*kernel)(A...), bool early, dim3 grid, int threads, cudaStream_t st, B... args) {
+static void launch_early(void (*kernel)(A...), bool early, dim3 grid, int threads, size_t smem, cudaStream_t st,
+                         B... args) {
   cudaLaunchAttribute at{};
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t c{};
   c.gridDim = grid;
   c.blockDim = dim3((unsigned)threads);
+  c.dynamicSmemBytes = smem;
   c.stream = st;
   c.attrs = &at;
   c.numAttrs = early ? 1 : 0;
   CK(cudaLaunchKernelEx(&c, kernel, static_cast<A>(args)...));
 }
 
+// The bottoms [first, end) of at most `rows` rows: the warps of a CTA share a bottom's edges, and a
+// CTA takes more groups one after another while there are CTAs enough.
+static void launch_bottom(const TreeArgs &a, bool early, int first, int end, int rows, cudaStream_t st) {
+  const int warps = std::min(kBottomWarps, a.ng);
+  int gpc = warps;
+  while (gpc < 64 && (int64_t)(end - first) * ((a.ng + 2 * gpc - 1) / (2 * gpc)) >= 148 * 24) gpc *= 2;
+  static_assert(kBottomWarps * kBottomRows * RowLayout::size <= 36 * 1024, "no opt-in for more than 48 KB");
+  const size_t smem = (size_t)warps * rows * RowLayout::size;
+  launch_early(k_bottom, early, dim3(end - first, (a.ng + gpc - 1) / gpc), warps * 32, smem, st, a, first, rows, gpc);
+}
+
 static void launch_bottoms(DeviceState *d, const TreeArgs &a, cudaStream_t st) {
   const TreePlan &p = *d->tree;
   if (a.ng > 4) {
+    // A launch runs into the tail of the one before it: all sources of 2k, 6k, 50k vertices 0.444 -> 0.394,
+    // 1.199 -> 1.125, 37.2 -> 36.4 ms, of a 5k core graph 2.00 -> 1.94.  A large core has so many bottoms that
+    // there is no tail to speak of, and the classes are better kept apart (200k + 2 %: 52.6 against 52.2 ms).
+    const bool overlap = p.core.nc < kCoreSmall;
     for (const TreePlan::BotClass &c : p.bot_class) {
-      launch_bottom(a, c.first, c.end, c.rows, st);
+      launch_bottom(a, overlap && &c != &p.bot_class.front(), c.first, c.end, c.rows, st);
       CK(cudaGetLastError());
       d->launches++;
     }
   } else if (p.nbot) {
-    launch_bottom(a, 0, p.nbot, p.bot_class[0].rows, st);
+    launch_bottom(a, false, 0, p.nbot, p.bot_class[0].rows, st);
     CK(cudaGetLastError());
     d->launches++;
   }
@@ -2534,7 +2547,7 @@ void launch_tree(const Handle &h, DeviceState *d, const int32_t *d_src_tid, int3
     for (int l = 0; l < levels; l++) {
       const int32_t *c = p.level_class.data() + 4 * l;
       if ((int64_t)(c[3] - c[0]) * a.ng < kWideCtas) {
-        launch_early(k_trunk_down_narrow, l > 0, dim3(c[3] - c[0], a.ng), kPieceLen * 32, st, a, c[0]);
+        launch_early(k_trunk_down_narrow, l > 0, dim3(c[3] - c[0], a.ng), kPieceLen * 32, 0, st, a, c[0]);
         launched();
         continue;
       }
@@ -2560,7 +2573,7 @@ void launch_tree(const Handle &h, DeviceState *d, const int32_t *d_src_tid, int3
     for (int l = levels - 1; l >= 0; l--) {
       const int32_t *c = p.level_class.data() + 4 * l;
       if ((int64_t)(c[3] - c[0]) * a.ng < kWideCtas) {
-        launch_early(k_trunk_up_narrow, l < levels - 1, dim3(c[3] - c[0], a.ng), kPieceLen * 32, st, a, c[0]);
+        launch_early(k_trunk_up_narrow, l < levels - 1, dim3(c[3] - c[0], a.ng), kPieceLen * 32, 0, st, a, c[0]);
         launched();
         continue;
       }
