@@ -36,7 +36,7 @@
 // kernels leave their results unused, and the call is answered by the label kernels.
 //
 // All 50,175 sources of the 50k grid: 239.8 ms by the label kernels (label scan 142, dependency pass
-// 77, sorting and gaps), 38.3 ms so; 1,024 sources of 500k 150.8 and 22.1 ms, 6,083 of 6k 3.31 and 1.20.
+// 77, sorting and gaps), 38.1 ms so; 1,024 sources of 500k 150.8 and 22.1 ms, 6,083 of 6k 3.33 and 1.16.
 #include <cuda_runtime.h>
 
 #include <algorithm>
