@@ -3472,7 +3472,9 @@ bool check_err(DeviceState *d) {
                              : e == ERR_SWEEP_BOUND ? "device: shortest-path sweep ran past its pass bound"
                                                    : "device: kernel error word " + std::to_string(e));
   }
-  return w[1] != 0 && tree_disable(d);
+  if (w[1] == 0 || !tree_disable(d)) return false;
+  sweep_cache_free(d);  // captured sweeps with the plan's launches in them answer nothing any more
+  return true;
 }
 
 // ------------------------------------------------------------------------------- drivers

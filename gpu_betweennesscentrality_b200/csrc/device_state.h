@@ -182,7 +182,8 @@ DeviceState *need_dev(Handle &h);
 // frees the captured sweep graphs (they hold scratch pointers; called whenever scratch changes)
 void sweep_cache_free(DeviceState *d);
 // reads and clears the device error word; throws QBC_EDEVICE when a kernel set it (synchronous).
-// True when a path count wrapped in a tree sweep since the last call: its results are void.
+// True when a path count wrapped in a tree sweep since the last call: its results are void, the plan
+// is given up, and the captured sweeps are gone (a caller holds no reference to one across this).
 bool check_err(DeviceState *d);
 
 }  // namespace qbc

@@ -60,7 +60,7 @@ uint64_t fnv(uint64_t h, const void *p, size_t bytes) {
 
 uint64_t tuning_key(const Handle &h, const DeviceState *d) {
   const Tuning &t = h.tuning;
-  const int32_t f[] = {t.lanes_per_source, t.label_threads, t.split, t.dep_threads, t.dep_form, t.queue_depth, t.label_warps, t.label_tile, t.label_passes, t.sweep_delta, t.sweep_threads, t.label_sources, t.label_stream, d->chunk, d->tree ? 1 : 0};
+  const int32_t f[] = {t.lanes_per_source, t.label_threads, t.split, t.dep_threads, t.dep_form, t.queue_depth, t.label_warps, t.label_tile, t.label_passes, t.sweep_delta, t.sweep_threads, t.label_sources, t.label_stream, d->chunk};
   return fnv(1469598103934665603ull, f, sizeof(f));
 }
 
@@ -161,14 +161,6 @@ void sweep_cache_free(DeviceState *d) {
   d->sweep = nullptr;
 }
 
-// Whether a path count of the sweep just finished wrapped: its captured graphs then go, and the
-// call is repeated with the label kernels.
-static bool sweep_wrapped(DeviceState *d) {
-  if (!check_err(d)) return false;
-  sweep_cache_free(d);
-  return true;
-}
-
 static constexpr size_t kMaxPlans = 4;
 
 static SweepPlan &plan_for(Handle &h, DeviceState *d, const int32_t *sources0, int32_t ns) {
@@ -178,6 +170,9 @@ static SweepPlan &plan_for(Handle &h, DeviceState *d, const int32_t *sources0, i
   uint64_t key = tuning_key(h, d);
   key = fnv(key, tids.data(), tids.size() * 4);
   key = fnv(key, &d->chunk, 4);
+  // which kernels it holds: a plan may be given up between two calls with the same list
+  const bool tree = use_tree(h, d, (int32_t)tids.size(), true);
+  key = fnv(key, &tree, sizeof(tree));
   for (size_t i = 0; i < c.plans.size(); i++)
     if (c.plans[i]->key == key && c.plans[i]->ns == (int32_t)tids.size()) {
       std::unique_ptr<SweepPlan> p = std::move(c.plans[i]);
@@ -222,7 +217,7 @@ void host_bc_sweep(Handle &h, const int32_t *sources0, int32_t ns, double *bc_ou
     launch_tid_to_vid(d, d->bc_tid, d->bc_vid, 0, st);
     CK(cudaMemcpyAsync(bc_out, d->bc_vid, (size_t)d->n * 8, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
-  } while (sweep_wrapped(d));
+  } while (check_err(d));
 }
 
 void host_query_batch(Handle &h, const int32_t *points0, int64_t total, const int32_t *sources0, int32_t ns, double *out) {
@@ -255,7 +250,7 @@ void host_query_batch(Handle &h, const int32_t *points0, int64_t total, const in
       CK(cudaMemcpyAsync(out, c.d_out, (size_t)total * 8, cudaMemcpyDeviceToHost, st));
     }
     CK(cudaStreamSynchronize(st));
-  } while (sweep_wrapped(d));
+  } while (check_err(d));
 }
 
 // ------------------------------------------------------------------------------- autotune

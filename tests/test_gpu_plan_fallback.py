@@ -1,0 +1,102 @@
+"""GPU: one index, several entry points, and an elimination-tree or core-graph plan that is given up
+between them (a path count past 2^31, a core distance from 2^25 on).  A call that was captured while
+the plan was in use has to be answered as before, by the label or sweep kernels."""
+import numpy as np
+import pytest
+
+import gpu_betweennesscentrality_b200 as Q
+import pyoracle as O
+from conftest import rel_err
+from util import BC_RTOL, lines_of, unit_grid_lines
+
+pytestmark = pytest.mark.gpu
+
+
+def _far_lines(blocks=40, step=1000000):
+    """Cliques of seven, a leaf at each vertex, in a chain with long links: the core is the cliques;
+    from the ends distances reach 39M, from the middle 20M, either side of 2^25"""
+    rng, e = np.random.default_rng(6), []
+    for b in range(blocks):
+        c = range(14 * b, 14 * b + 7)
+        e += [(i, j, int(rng.integers(1, 9))) for i in c for j in range(14 * b, i)]
+        e += [(i, i + 7, int(rng.integers(1, 9))) for i in c]
+        if b:
+            e.append((14 * b, 14 * b - 13, step))
+    return lines_of(e, 14 * blocks)
+
+
+def _far():
+    """label-free index: harmless sources, sources that give the plan up"""
+    n, u, v, w = _far_lines()
+    g = Q.Graph(device=0)
+    g.ReadLines(n, u, v, w)
+    middle = np.arange(n // 2 - 20, n // 2 + 20, dtype=np.int32)
+    return n, O.Arcs(n, u, v, w), g.build_index(Q.QBC_INDEX_CSR), middle, np.arange(12, dtype=np.int32)
+
+
+def _unit_grid():
+    """H2H index of the 24 x 24 unit grid: counts from its middle end at C(24, 12), from a corner pass 2^31"""
+    n, u, v, w = unit_grid_lines()
+    g = Q.Graph(device=0)
+    g.ReadLines(n, u, v, w)
+    idx = g.build_index(Q.QBC_INDEX_H2H, g.min_degree_order(), on_device=True)
+    middle = np.array([24 * r + c for r in (11, 12) for c in (11, 12)], np.int32)
+    return n, O.Arcs(n, u, v, w), idx, middle, np.arange(24, dtype=np.int32)
+
+
+def _device_call(idx, n, srcs):
+    import torch
+
+    d_src = torch.from_numpy(srcs).cuda()
+    d_bc = torch.zeros(n, dtype=torch.float64, device="cuda:0")
+    torch.cuda.synchronize()
+    idx.bc_sources_device(d_src.data_ptr(), len(srcs), d_bc.data_ptr())
+    torch.cuda.synchronize()
+    return d_bc.cpu().numpy()
+
+
+BETWEEN = {
+    "sources": lambda idx, n, middle, void: idx.bc_sources(void),
+    "device_rows": lambda idx, n, middle, void: (_device_call(idx, n, void), idx.rows(middle[:2])),
+    "device_plain": lambda idx, n, middle, void: (_device_call(idx, n, void), idx.bc_plain(middle[:2])),
+    "device_only": lambda idx, n, middle, void: _device_call(idx, n, void),
+    "query": lambda idx, n, middle, void: idx.bc_query_batch([middle], void),
+    "autotune": lambda idx, n, middle, void: idx.autotune(void),
+}
+
+
+@pytest.mark.parametrize("between", sorted(BETWEEN))
+@pytest.mark.parametrize("make", [_far, _unit_grid])
+def test_captured_call_after_the_plan_is_given_up(make, between, monkeypatch):
+    monkeypatch.setenv("QBC_TREE_MIN_PAIRS", "0")
+    n, arcs, idx, middle, void = make()
+    sets = [np.arange(0, n, 3, dtype=np.int32), np.arange(n, dtype=np.int32)]
+    want = arcs.bc(middle)
+    assert want.any()
+
+    def answered():
+        """right twice (captured, then replayed), and with how many launches"""
+        for _ in range(2):
+            idx.profile(True)
+            for s, got in zip(sets, idx.bc_query_batch(sets, middle)):
+                assert rel_err(got, want[s]) <= BC_RTOL
+        return idx.stats()["launches"]
+
+    with_plan = answered()
+    BETWEEN[between](idx, n, middle, void)
+    assert answered() != with_plan
+    assert rel_err(idx.bc_sources(middle), want) <= BC_RTOL
+
+
+def test_captured_call_after_the_threshold_moves(monkeypatch):
+    """a graph captured with the tree's launches is not the one for a call that the rule sends elsewhere"""
+    n, arcs, idx, middle, _ = _unit_grid()
+    want = arcs.bc(middle)
+    launches = []
+    for pairs in ("0", "1000000000", "0"):
+        monkeypatch.setenv("QBC_TREE_MIN_PAIRS", pairs)
+        idx.bc_query_batch([middle], middle)  # captures
+        idx.profile(True)
+        assert rel_err(idx.bc_query_batch([middle], middle)[0], want[middle]) <= BC_RTOL
+        launches.append(idx.stats()["launches"])
+    assert launches[0] == launches[2] != launches[1]
