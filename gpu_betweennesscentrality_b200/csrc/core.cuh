@@ -502,8 +502,8 @@ __global__ void k_core_src(const int32_t *__restrict__ tid, const int32_t *__res
 }
 
 __global__ void k_core_finish(const double *__restrict__ F, const int32_t *__restrict__ cid_of, double *__restrict__ bc_tid, int n,
-                              const int32_t *wrap) {
-  if (__ldcg(wrap) != 0) return;
+                              const int32_t *err) {
+  if (result_void(err)) return;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t < n) bc_tid[t] += 0.5 * F[cid_of[t]];
 }

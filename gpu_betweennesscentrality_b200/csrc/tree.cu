@@ -1595,8 +1595,13 @@ __global__ void __cluster_dims__(kTailCtas, 1, 1) __launch_bounds__(1024)
   }
 }
 
-__global__ void k_finish(const double *__restrict__ F, double *__restrict__ bc_tid, int n, const int32_t *wrap) {
-  if (__ldcg(wrap) != 0) return;
+// The result of a call is left out where its counts wrapped, and where the error word is set (a source
+// id out of range, read here as vertex 0): the call reports that, and the caller's BC stays as it was, as
+// with the dependency kernels (see rows_failed).  err: the error word, then the wrap word.
+__device__ __forceinline__ bool result_void(const int32_t *err) { return __ldcg(err) != ERR_NONE || __ldcg(err + 1) != 0; }
+
+__global__ void k_finish(const double *__restrict__ F, double *__restrict__ bc_tid, int n, const int32_t *err) {
+  if (result_void(err)) return;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) bc_tid[t] += 0.5 * F[t];
 }
 
@@ -2494,7 +2499,7 @@ static void launch_core(const Handle &h, DeviceState *d, const int32_t *d_src_ti
     d->dep_launches++;
   }
   launch_unpack(d, st);
-  k_core_finish<<<blocks_for(p.args.n, 256), 256, 0, st>>>(p.args.F, p.cid_of, d->bc_tid, p.args.n, p.args.wrap);
+  k_core_finish<<<blocks_for(p.args.n, 256), 256, 0, st>>>(p.args.F, p.cid_of, d->bc_tid, p.args.n, d->err);
   launched();
 }
 
@@ -2602,7 +2607,7 @@ void launch_tree(const Handle &h, DeviceState *d, const int32_t *d_src_tid, int3
     d->dep_launches++;
   }
   launch_unpack(d, st);
-  k_finish<<<std::min(148 * 4, (p.args.n + 255) / 256), 256, 0, st>>>(p.args.F, d->bc_tid, p.args.n, p.args.wrap);
+  k_finish<<<std::min(148 * 4, (p.args.n + 255) / 256), 256, 0, st>>>(p.args.F, d->bc_tid, p.args.n, d->err);
   launched();
 }
 

@@ -1,13 +1,14 @@
-"""GPU: one index, several entry points, and an elimination-tree or core-graph plan that is given up
-between them (a path count past 2^31, a core distance from 2^25 on).  A call that was captured while
-the plan was in use has to be answered as before, by the label or sweep kernels."""
+"""GPU: what a call over an elimination-tree or core-graph plan leaves behind.  One index, several
+entry points, and a plan that is given up between them (a path count past 2^31, a core distance from
+2^25 on): a call that was captured while the plan was in use has to be answered as before, by the label
+or sweep kernels.  And a source id out of range in a device list, which only the device can find."""
 import numpy as np
 import pytest
 
 import gpu_betweennesscentrality_b200 as Q
 import pyoracle as O
 from conftest import rel_err
-from util import BC_RTOL, lines_of, unit_grid_lines
+from util import BC_RTOL, grid_lines, lines_of, unit_grid_lines
 
 pytestmark = pytest.mark.gpu
 
@@ -100,3 +101,30 @@ def test_captured_call_after_the_threshold_moves(monkeypatch):
         assert rel_err(idx.bc_query_batch([middle], middle)[0], want[middle]) <= BC_RTOL
         launches.append(idx.stats()["launches"])
     assert launches[0] == launches[2] != launches[1]
+
+
+@pytest.mark.parametrize("bad", [-1, "n"])
+@pytest.mark.parametrize("kind", [Q.QBC_INDEX_MHL, Q.QBC_INDEX_H2H, Q.QBC_INDEX_CSR])
+def test_bad_device_source_leaves_the_vector(kind, bad, monkeypatch):
+    """an id out of range is found on the device: nothing is added, the next host call reports it, the
+    one after that is right"""
+    import torch
+
+    monkeypatch.setenv("QBC_TREE_MIN_PAIRS", "0")
+    n, u, v, w = grid_lines(1500, seed=5, shortcut_frac=0.02 if kind == Q.QBC_INDEX_CSR else 0.0)
+    g = Q.Graph(device=0)
+    g.ReadLines(n, u, v, w)
+    idx = g.build_index(kind, g.min_degree_order() if kind == Q.QBC_INDEX_H2H else None, on_device=True)
+    srcs = np.arange(0, n, 9, dtype=np.int32)
+    with_bad = srcs.copy()
+    with_bad[7] = n if bad == "n" else bad
+    before = np.arange(n, dtype=np.float64)
+    d_bc = torch.from_numpy(before).cuda()
+    d_src = torch.from_numpy(with_bad).cuda()
+    torch.cuda.synchronize()
+    idx.bc_sources_device(d_src.data_ptr(), len(srcs), d_bc.data_ptr())
+    torch.cuda.synchronize()
+    assert np.array_equal(d_bc.cpu().numpy(), before)
+    with pytest.raises(Q.QbcError, match="out of range"):
+        idx.bc_sources(srcs)
+    assert rel_err(idx.bc_sources(srcs), O.Arcs(n, u, v, w).bc(srcs)) <= BC_RTOL
