@@ -529,7 +529,7 @@ static void core_ranges(int32_t count, F &&f) {
   for (std::thread &t : ts) t.join();
 }
 
-// The elimination; false where no plan is possible (a count past 2^31, a degree past the sweep's, or
+// The elimination, of paired arcs (Index::arcs_paired); false where no plan is possible (a count past 2^31, a degree past the sweep's, or
 // lengths below 1, which a graph has none of but a file might).
 static bool core_shape(const Index &ix, CoreShape &s) {
   const int32_t n = ix.n;

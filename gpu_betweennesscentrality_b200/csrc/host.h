@@ -97,6 +97,9 @@ struct Index {
   int32_t max_label = 0;         // largest label distance (decides the packed-key scan)
   // arcs in tid space, each tail's arcs in file order
   std::vector<int32_t> arc_off, arc_head, arc_w;
+  // every arc has its reverse of the same weight, no head is listed twice, none is its own tail: the
+  // graph reader sees to that, a file need not (looked at when a CSR index is loaded)
+  bool arcs_paired = true;
   int64_t depth_sum = 0;
   Separators seps;           // empty for an index loaded from a file (and for CSR)
   bool counts_wrapped = false;  // a label's path count passed 2^31 when the rows were filled

@@ -19,6 +19,8 @@
 #include <cstdio>
 #include <cstring>
 #include <memory>
+#include <utility>
+#include <vector>
 
 #include "../../include/qbc_b200.h"
 #include "host.h"
@@ -120,6 +122,30 @@ struct File {
     get(v.data(), count * sizeof(T));
   }
 };
+
+// Index::arcs_paired.  The reversed arcs are bucketed by their tails in increasing order of their
+// heads, so each vertex's own arcs, sorted, must be its bucket.
+bool arcs_paired(const Index &ix) {
+  const size_t n = (size_t)ix.n;
+  std::vector<int32_t> next(n, 0);
+  for (int32_t h : ix.arc_head) next[h]++;
+  for (size_t v = 0; v < n; v++) {
+    if (next[v] != ix.arc_off[v + 1] - ix.arc_off[v]) return false;  // as many in as out
+    next[v] = ix.arc_off[v];
+  }
+  std::vector<std::pair<int32_t, int32_t>> in(ix.arc_head.size()), out;
+  for (int32_t v = 0; v < ix.n; v++)
+    for (int32_t q = ix.arc_off[v]; q < ix.arc_off[v + 1]; q++) in[next[ix.arc_head[q]]++] = {v, ix.arc_w[q]};
+  for (int32_t v = 0; v < ix.n; v++) {
+    const int32_t b = ix.arc_off[v], e = ix.arc_off[v + 1];
+    out.clear();
+    for (int32_t q = b; q < e; q++) out.push_back({ix.arc_head[q], ix.arc_w[q]});
+    std::sort(out.begin(), out.end());
+    for (int32_t q = b; q < e; q++)
+      if (in[q] != out[q - b] || in[q].first == v || (q > b && in[q].first == in[q - 1].first)) return false;
+  }
+  return true;
+}
 
 }  // namespace
 
@@ -223,6 +249,7 @@ Index index_load(const std::string &path) {
   }
   for (int32_t hd : ix.arc_head)
     if (hd < 0 || hd >= ix.n) throw Error(QBC_EIO, path + ": inconsistent index arrays");
+  if (csr) ix.arcs_paired = arcs_paired(ix);
   for (int32_t a : ix.anc)
     if (a < 0 || a >= ix.n) throw Error(QBC_EIO, path + ": inconsistent index arrays");
   ix.rows_on_host = true;

@@ -2187,6 +2187,7 @@ void core_build(Handle &h, DeviceState *d) {
   constexpr uint32_t lim = 1u << (32 - bits);
   const int32_t lcap = (int32_t)(lim / (4 * kCoreChain));
   CoreShape s;
+  if (!ix.arcs_paired) return;  // the elimination finds an arc's reverse; the sweep of the whole graph answers
   if (!core_shape(ix, s) || (int64_t)s.nc * 4 > (int64_t)n * 3) return;  // (a core that is most of the graph saves nothing)
   if ((size_t)core_words(s.nc) * 8 + 8192 > (size_t)d->smem_optin) return;  // its list bits are in shared memory
   for (size_t e = (size_t)s.xoff[s.nc]; e < s.eL.size(); e++)
