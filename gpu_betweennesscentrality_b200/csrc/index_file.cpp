@@ -234,7 +234,8 @@ Index index_load(const std::string &path) {
   uint64_t sum = 0;
   if (std::fread(&sum, 8, 1, f.f) != 1 || sum != want) throw Error(QBC_EIO, path + ": index file checksum mismatch");
   // structural checks the kernels rely on
-  if (ix.lab_off[n] != L || ix.arc_off[n] != arcs) throw Error(QBC_EIO, path + ": inconsistent index arrays");
+  if (ix.lab_off[0] != 0 || ix.arc_off[0] != 0 || ix.lab_off[n] != L || ix.arc_off[n] != arcs)
+    throw Error(QBC_EIO, path + ": inconsistent index arrays");
   for (size_t t = 0; t < n && csr; t++) {
     if (ix.depth[t] != 0 || ix.parent[t] != -1 || ix.send[t] != (int32_t)t + 1 || ix.lab_off[t] != 0 ||
         ix.vid_of[t] < 0 || ix.vid_of[t] >= ix.n || ix.tid_of[ix.vid_of[t]] != (int32_t)t || ix.arc_off[t] > ix.arc_off[t + 1])

@@ -8,7 +8,7 @@ import numpy as np
 import pytest
 
 import gpu_betweennesscentrality_b200 as Q
-from gpu_betweennesscentrality_b200 import build
+from gpu_betweennesscentrality_b200 import build, capi
 from test_index_file import _word_hash
 from util import grid_lines
 
@@ -100,6 +100,18 @@ def test_unpaired_arcs_are_marked(saved, paired, tmp_path, edit):
     bad = _edited(saved, str(tmp_path / "bad.qbcidx"), edit)
     assert paired(saved[0], bad) == [True, False]
     assert Q.Index.load(bad, device=None).n == saved[1]  # accepted as before
+
+
+@pytest.mark.parametrize("first", [-1, 1])
+def test_arcs_that_do_not_start_at_0_are_refused(saved, tmp_path, first):
+    p, n, off, at, arcs = saved
+    raw = bytearray(open(p, "rb").read()[:-8])
+    np.frombuffer(raw, np.int32, n + 1, at - 4 * (n + 1))[0] = first
+    bad = str(tmp_path / "bad.qbcidx")
+    open(bad, "wb").write(bytes(raw) + _word_hash(bytes(raw)).to_bytes(8, "little"))
+    with pytest.raises(Q.QbcError) as e:
+        Q.Index.load(bad, device=None)
+    assert e.value.code == capi.QBC_EIO
 
 
 def test_every_recipe_is_paired(paired, tmp_path):
