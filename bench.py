@@ -312,7 +312,8 @@ def label_roofline(idx, shard, n, stats, steps, peak, peak_src, sm_mhz):
     algorithmic figure of the workload's byte model (12 B per label entry scanned + 12 B per pair)
     is given as effective_bw: rows are reused by every source of a group, so it exceeds the HBM
     peak."""
-    if not any(idx.get_tuning().get(k) for k in LABEL_FIELDS):
+    tuning = idx.get_tuning()
+    if tuning.get("keep_plan") or not any(tuning.get(k) for k in LABEL_FIELDS):
         return tree_roofline(idx, shard, n, stats, steps, peak, peak_src)
     ns = len(shard)
     per_cta = idx.label_group() or 32

@@ -49,7 +49,7 @@ void need(bool ok, const char *what) {
   if (!ok) throw qbc::Error(QBC_EINVAL, what);
 }
 
-constexpr int32_t kTuningFields = 14;  // qbc_index_set_tuning's params layout
+constexpr int32_t kTuningFields = 15;  // qbc_index_set_tuning's params layout
 
 void not_serving(const qbc_index *idx) {
   if (idx->h.server) throw qbc::Error(QBC_EBUSY, "the index is serving requests: close its server first");
@@ -294,7 +294,7 @@ int qbc_index_set_tuning(qbc_index *idx, const int32_t *params, int32_t nparams)
     need(idx && (nparams == 0 || params), "null argument");
     qbc::Tuning &t = idx->h.tuning;
     not_serving(idx);
-    int32_t *f[] = {&t.lanes_per_source, &t.label_threads, &t.split, &t.chunk, &t.dep_threads, &t.dep_form, &t.queue_depth, &t.label_warps, &t.label_tile, &t.label_passes, &t.sweep_delta, &t.sweep_threads, &t.label_sources, &t.label_stream};
+    int32_t *f[] = {&t.lanes_per_source, &t.label_threads, &t.split, &t.chunk, &t.dep_threads, &t.dep_form, &t.queue_depth, &t.label_warps, &t.label_tile, &t.label_passes, &t.sweep_delta, &t.sweep_threads, &t.label_sources, &t.label_stream, &t.keep_plan};
     if (nparams > 0) {
       int32_t k = params[0];
       need(k == 0 || k == 1 || k == 2 || k == 4 || k == 8 || k == 16 || k == 32, "lanes per source must be 0 or a power of two <= 32");
@@ -313,6 +313,8 @@ int qbc_index_set_tuning(qbc_index *idx, const int32_t *params, int32_t nparams)
            "sweep threads must be 0, 256, 512, 1024 or 2048 (four 512-thread CTAs per SM)");
     if (nparams > 12) need(params[12] == 0 || params[12] == 16 || params[12] == 32, "label sources must be 0, 16 or 32");
     if (nparams > 13) need(params[13] >= 0 && params[13] <= 2, "label stream must be 0, 1 or 2");
+    if (nparams > 14) need(params[14] == 0 || params[14] == 1, "keep plan must be 0 or 1");
+    if (nparams > 0) t.keep_plan = 0;  // (unless the list reaches it: shorter ones mean what they always did)
     for (int32_t i = 0; i < nparams && i < kTuningFields; i++) *f[i] = params[i];
     if (nparams > 3 && t.chunk != old_chunk && idx->h.dev) qbc::device_set_chunk(idx->h, t.chunk);
   });
@@ -322,7 +324,7 @@ int qbc_index_get_tuning(const qbc_index *idx, int32_t *params, int32_t nparams)
   return guarded([&] {
     need(idx && (nparams == 0 || params), "null argument");
     const qbc::Tuning &t = idx->h.tuning;
-    const int32_t f[] = {t.lanes_per_source, t.label_threads, t.split, t.chunk, t.dep_threads, t.dep_form, t.queue_depth, t.label_warps, t.label_tile, t.label_passes, t.sweep_delta, t.sweep_threads, t.label_sources, t.label_stream};
+    const int32_t f[] = {t.lanes_per_source, t.label_threads, t.split, t.chunk, t.dep_threads, t.dep_form, t.queue_depth, t.label_warps, t.label_tile, t.label_passes, t.sweep_delta, t.sweep_threads, t.label_sources, t.label_stream, t.keep_plan};
     for (int32_t i = 0; i < nparams && i < kTuningFields; i++) params[i] = f[i];
   });
 }
@@ -411,7 +413,7 @@ int qbc_autotune(qbc_index *idx, const int32_t *sources0, int32_t ns, int32_t *p
     qbc::autotune(idx->h, sources0, ns, &ms);
     if (ms_per_source) *ms_per_source = ms;
     const qbc::Tuning &t = idx->h.tuning;
-    const int32_t f[] = {t.lanes_per_source, t.label_threads, t.split, t.chunk, t.dep_threads, t.dep_form, t.queue_depth, t.label_warps, t.label_tile, t.label_passes, t.sweep_delta, t.sweep_threads, t.label_sources, t.label_stream};
+    const int32_t f[] = {t.lanes_per_source, t.label_threads, t.split, t.chunk, t.dep_threads, t.dep_form, t.queue_depth, t.label_warps, t.label_tile, t.label_passes, t.sweep_delta, t.sweep_threads, t.label_sources, t.label_stream, t.keep_plan};
     for (int32_t i = 0; params && i < nparams && i < kTuningFields; i++) params[i] = f[i];
   });
 }

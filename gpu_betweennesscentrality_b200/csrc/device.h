@@ -27,6 +27,8 @@ struct Tuning {
                                  // tall trees in shared memory); 0 = auto
   int32_t label_stream = 0;      // 16-source kernel: 1 whole target rows double-buffered, 2 64-entry
                                  // blocks through a ring; 0 = auto (whole rows when they fit 16 warps)
+  int32_t keep_plan = 0;         // 1: the label and dependency fields configure those kernels for the calls
+                                 // that are too small for the elimination tree; 0: they ask for them in all
 };
 
 struct DeviceState;  // opaque, defined in device_state.h

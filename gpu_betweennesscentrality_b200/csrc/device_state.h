@@ -154,6 +154,8 @@ void tree_build(Handle &h, DeviceState *d, const std::vector<int64_t> &soff, con
 void core_build(Handle &h, DeviceState *d);  // the same for the label-free index (core.cuh)
 void tree_free(DeviceState *d);
 bool use_tree(const Handle &h, const DeviceState *d, int32_t ns, bool rerun);
+// the part of use_tree that no list's length changes: some list is answered by the plan
+bool plan_open(const Handle &h, const DeviceState *d);
 // k_src_rows by the plan's runs of ancestors; false without a plan
 bool tree_source_rows(const DeviceState *d, const int32_t *src, int32_t ns, int32_t stride, int32_t *rows, cudaStream_t st);
 const int32_t *tree_guard(const DeviceState *d);

@@ -60,7 +60,7 @@ uint64_t fnv(uint64_t h, const void *p, size_t bytes) {
 
 uint64_t tuning_key(const Handle &h, const DeviceState *d) {
   const Tuning &t = h.tuning;
-  const int32_t f[] = {t.lanes_per_source, t.label_threads, t.split, t.dep_threads, t.dep_form, t.queue_depth, t.label_warps, t.label_tile, t.label_passes, t.sweep_delta, t.sweep_threads, t.label_sources, t.label_stream, d->chunk};
+  const int32_t f[] = {t.lanes_per_source, t.label_threads, t.split, t.dep_threads, t.dep_form, t.queue_depth, t.label_warps, t.label_tile, t.label_passes, t.sweep_delta, t.sweep_threads, t.label_sources, t.label_stream, t.keep_plan, d->chunk};
   return fnv(1469598103934665603ull, f, sizeof(f));
 }
 
@@ -302,6 +302,10 @@ void autotune(Handle &h, const int32_t *sources0, int32_t ns, double *ms_per_sou
     const int32_t cnt = (int32_t)tids.size();
     Tuning best = h.tuning;
     double best_t = time_sample(h, d, d_tids, cnt, 3);
+    // A list that is too short for the elimination tree times the label kernels; what wins there is kept
+    // for such lists, and longer ones stay with the tree (50k, tuned on 16 sources: those 0.84 -> 0.63 ms,
+    // all sources 38 ms instead of the 230 of the label kernels).
+    const bool short_list = plan_open(h, d) && !use_tree(h, d, cnt, false);
     auto trial = [&](const Tuning &t) {
       h.tuning = t;
       try {
@@ -355,6 +359,11 @@ void autotune(Handle &h, const int32_t *sources0, int32_t ns, double *ms_per_sou
       cudaFree(d_tids);
       return;
     }
+    auto label_trial = [&] {
+      Tuning t = best;
+      t.keep_plan = short_list;
+      return t;
+    };
     // 1. label kernel: the packed-key kernel with 32 sources per CTA and 8-20 warps (0 lanes) and,
     //    for tall trees, tile passes or a global-memory tail; its 16-source forms (whole source rows
     //    in shared memory, two targets per warp; target rows whole or through a ring) with 8, 12 or
@@ -364,7 +373,7 @@ void autotune(Handle &h, const int32_t *sources0, int32_t ns, double *ms_per_sou
       for (int32_t warps : {8, 12, 16, 20})  // 12: the two-target kernel
         for (int32_t passes : {0, 2}) {  // rows taller than a 16-warp tile: global tail or tile passes
           if (passes == 2 && (d->hmax_pad <= 644 || warps == 12)) continue;
-          Tuning t = best;
+          Tuning t = label_trial();
           t.lanes_per_source = 0;
           t.label_sources = 32;
           t.label_warps = warps;
@@ -373,7 +382,7 @@ void autotune(Handle &h, const int32_t *sources0, int32_t ns, double *ms_per_sou
         }
       for (int32_t stream : {1, 2})
         for (int32_t warps : {8, 12, 16}) {
-          Tuning t = best;
+          Tuning t = label_trial();
           t.lanes_per_source = 0;
           t.label_sources = 16;
           t.label_stream = stream;
@@ -386,28 +395,28 @@ void autotune(Handle &h, const int32_t *sources0, int32_t ns, double *ms_per_sou
     for (int32_t lanes : {4, 8, 16})
       for (int32_t threads : {128, 256}) {
         if (!label_fits(h, d, lanes, threads)) continue;
-        Tuning t = best;
+        Tuning t = label_trial();
         t.lanes_per_source = lanes;
         t.label_threads = threads;
         trial(t);
       }
     // 2. target ranges per source group (the width of each CTA's target tile)
     for (int32_t split : {0, 2, 4, 8, 16, 32}) {
-      Tuning t = best;
+      Tuning t = label_trial();
       t.split = split;
       trial(t);
     }
     // 3. dependency pass: warp per source with its shared level-queue depth, or CTA per source
     for (int32_t form : {1, 3})
       for (int32_t qd : {64, 256, 512, 1024}) {
-        Tuning t = best;
+        Tuning t = label_trial();
         t.dep_form = form;
         t.queue_depth = qd;
         trial(t);
       }
     for (int32_t form : {2, 4})
       for (int32_t th : {128, 256}) {
-        Tuning t = best;
+        Tuning t = label_trial();
         t.dep_form = form;
         t.dep_threads = th;
         trial(t);

@@ -2304,16 +2304,20 @@ static int64_t min_pairs(const Handle &h, bool rerun) {
   return rerun ? std::max<int64_t>(0, 3600000 - 68 * (int64_t)h.host.n) : 2 << 20;
 }
 
-bool use_tree(const Handle &h, const DeviceState *d, int32_t ns, bool rerun) {
+bool plan_open(const Handle &h, const DeviceState *d) {
   const Tuning &t = h.tuning;
-  if (!d->tree || d->tree->off || ns < 1) return false;
+  if (!d->tree || d->tree->off) return false;
   // a tuning that picks a label or dependency kernel, or the test hook of the label rows' copies, gets it
-  if (t.lanes_per_source || t.split || t.dep_form || t.queue_depth || t.label_warps || t.label_tile || t.label_passes ||
-      t.label_sources || t.label_stream)
+  if (!t.keep_plan && (t.lanes_per_source || t.split || t.dep_form || t.queue_depth || t.label_warps || t.label_tile ||
+                       t.label_passes || t.label_sources || t.label_stream))
     return false;
   const char *hook = std::getenv("QBC_TEST_ROW_WAIT_SPINS");
   if (hook && *hook) return false;
-  return (int64_t)ns * d->n >= min_pairs(h, rerun) && groups_fit(d) >= 1;
+  return groups_fit(d) >= 1;
+}
+
+bool use_tree(const Handle &h, const DeviceState *d, int32_t ns, bool rerun) {
+  return ns >= 1 && (int64_t)ns * d->n >= min_pairs(h, rerun) && plan_open(h, d);
 }
 
 bool tree_source_rows(const DeviceState *d, const int32_t *src, int32_t ns, int32_t stride, int32_t *rows, cudaStream_t st) {

@@ -142,9 +142,11 @@ int qbc_index_export(const qbc_index *idx, int32_t *vid_of, int32_t *depth, int3
  * shared memory, two targets per warp, target rows streamed through a cp.async ring, when the
  * height fits; 0 = auto: 16 when the 32-source kernel cannot hold whole rows and [7]-[9] are 0),
  * [13]=target rows of the 16-source kernel (1 = whole rows, double-buffered per warp side; 2 =
- * 64-entry blocks through a ring; 0 = auto: whole rows when they fit with 16 warps).  Refused
- * with QBC_EBUSY while the index serves.
- * With [0], [2], [5]-[9], [12] and [13] all 0, BC of many (source, vertex) pairs runs over the
+ * 64-entry blocks through a ring; 0 = auto: whole rows when they fit with 16 warps),
+ * [14]=1: [0], [2], [5]-[9], [12] and [13] configure the label kernels for the calls that are too
+ * small for the elimination tree (below) without asking for them in the others; a list of fewer
+ * params leaves it 0.  Refused with QBC_EBUSY while the index serves.
+ * With [0], [2], [5]-[9], [12] and [13] all 0, or [14] 1, BC of many (source, vertex) pairs runs over the
  * elimination tree (label indexes built here, not loaded from a file) or over the core graph (CSR
  * index; [10] and [11] apply, [11] = 0 chooses by the core's size) instead of the label, sweep and
  * dependency kernels; any of those fields set asks for the latter.  A path count past 2^31 does, too,
@@ -163,10 +165,10 @@ int qbc_index_stats(qbc_index *idx, double *out);
 /* Autotuner (no counterpart in the reference): times candidate tunings -- sources per CTA and
  * threads of the label kernel, target split, dependency form and level-queue depth, chunk size --
  * on a sweep over the listed sources, keeps the fastest on the index and returns it in params
- * (layout of qbc_index_set_tuning, up to 12) with its time per source in ms.  On a CSR index
- * it tunes the sweep's bucket width and threads, the dependency threads and the chunk size.  Tune on a
- * list as long as those to come: a short one is answered by the label kernels, and the fields that it
- * then sets keep them. */
+ * (layout of qbc_index_set_tuning, up to 15) with its time per source in ms.  On a CSR index
+ * it tunes the sweep's bucket width and threads, the dependency threads and the chunk size.  A list
+ * too short for the elimination tree tunes the label kernels for such lists, with [14] set: keep that
+ * field, too, where the params are kept to be set again. */
 int qbc_autotune(qbc_index *idx, const int32_t *sources0, int32_t ns, int32_t *params, int32_t nparams,
                  double *ms_per_source);
 

@@ -128,3 +128,37 @@ def test_bad_device_source_leaves_the_vector(kind, bad, monkeypatch):
     with pytest.raises(Q.QbcError, match="out of range"):
         idx.bc_sources(srcs)
     assert rel_err(idx.bc_sources(srcs), O.Arcs(n, u, v, w).bc(srcs)) <= BC_RTOL
+
+
+def _launches(idx, call):
+    call()  # captures
+    idx.profile(True)
+    call()
+    return idx.stats()["launches"]
+
+
+def test_autotune_on_a_short_list_keeps_the_plan_for_longer_ones(tmp_path):
+    n, u, v, w = grid_lines(6007, seed=3)
+    g = Q.Graph(device=0)
+    g.ReadLines(n, u, v, w)
+    idx = g.build_index(on_device=True)
+    few = np.arange(5, n, n // 15, dtype=np.int32)
+    all_tree, want = _launches(idx, idx.bc_all), idx.bc_all()
+    few_want = O.Arcs(n, u, v, w).bc(few)
+    path = str(tmp_path / "tuning.json")
+    idx.autotune(few, path=path)
+    assert _launches(idx, idx.bc_all) == all_tree
+    assert rel_err(idx.bc_all(), want) <= BC_RTOL
+    assert rel_err(idx.bc_sources(few), few_want) <= BC_RTOL
+    idx.set_tuning()
+    idx.load_tuning(path)
+    assert _launches(idx, idx.bc_all) == all_tree
+    idx.set_tuning(label_sources=16, label_warps=16, label_stream=1, keep_plan=1)
+    assert _launches(idx, idx.bc_all) == all_tree and idx.label_group() == 16
+    assert rel_err(_device_call(idx, n, few), few_want) <= BC_RTOL
+    idx.set_tuning(label_sources=16, label_warps=16, label_stream=1)
+    assert _launches(idx, idx.bc_all) != all_tree
+    idx.set_tuning()
+    idx.autotune(np.arange(0, n, 3, dtype=np.int32))  # long enough for the tree: it wins
+    t = idx.get_tuning()
+    assert t["keep_plan"] == t["label_warps"] == t["split"] == t["dep_form"] == 0
