@@ -2286,22 +2286,49 @@ static int groups_fit(const DeviceState *d) {
   return (int)fit;
 }
 
-// (source, vertex) pairs from which the tree is the faster path.  Its launches follow the trunk level by
-// level, however few the sources: 0.24, 0.31, 0.47, 0.78, 1.5 and 5.1 ms for one source of 2k, 6k, 21k,
-// 50k, 120k and 500k vertices.  The label kernels of an MHL index start lower on small graphs and rise
-// with the pairs: 0.15, 0.18, 0.33, 0.63, 1.5, 5.2 ms for one source, and the two meet at about 3.3M
-// pairs (6k: 0.492 against 0.457 ms at 3.1M), 2.2M (12k), 1.5M (21k) and 0.2M (50k: 0.820 against
-// 0.839 ms at 4 sources); a line through those.  Calls that only enqueue are followed by the guarded
-// label launches and often overlap with others, where the tree's chain has little to offer: 2M for
-// those.  An H2H index counts paths by Kahn waves on the label path, which is slower from the first
-// source on (1,023 vertices 0.196 against 0.244 ms, 21k 0.59 against 1.47).  QBC_TREE_MIN_PAIRS overrides
-// it for tests.
+// (source, vertex) pairs from which the plan is the faster path.
+//
+// MHL: the tree's launches follow the trunk level by level, however few the sources (0.36, 0.43, 0.59, 0.85,
+// 1.5 and 5.1 ms for a few sources of 2k, 6k, 21k, 50k, 120k and 500k vertices); the label kernels start
+// lower on graphs up to 80k vertices and rise with the pairs.  Time of the tree over that of the label
+// kernels, grids of three seeds, calls that wait for their result: 6k vertices 1.11 at 1.5M pairs, 1.10 at
+// 2M, 0.97 at 2.75M, 0.91 at 3M; 21k 1.09 at 1.25M, 0.98 at 1.75M; 45k 1.17 at 0.4M, 1.06 at 1.25M, 0.95 at
+// 1.5M; 70k 1.03 at 0.2M, 0.97 at 0.8M; 90k to 160k below 1 from the first source; 200k to 350k 0.93 to 1.12
+// (1.05 on average) for one source, 0.95 for two.  The lines below join the sizes' crossings, which lie at 1.8M (1.5k), 2.1M (2k), 3.0M (4k),
+// 2.7M (6k), 3.2M (8k), 2.4M (12k), 2.1M (16k), 1.8M (21k), 1.4M (30k to 60k) and 0.6M (70k).  (A line from
+// 3.6M falling by 68 per vertex cost calls of 30k to 60k vertices up to a fifth.)
+// Calls that only enqueue are followed by the guarded label launches: crossings at 2.0M (1.5k), 2.3M (2k),
+// 3.4M (4k), 2.8M (6k), 3.4M (8k), 2.6M (12k), 2.3M (16k), 2.0M (21k).  (2M for all sizes: 333 sources of 6k
+// 0.36 ms, by the label kernels 0.29.)  From 21k vertices on such calls often overlap with others, where the
+// tree's chain has little to offer: 2M.
+//
+// H2H: the label path counts paths by Kahn waves and is slower from the first source on (1,023 vertices
+// 0.194 against 0.241 ms, 20k 0.62 against 1.29).
+//
+// Label-free: the core from the first source on (one source of 100 vertices 0.163 against 0.177 ms, 400
+// 0.19 and 0.27, 5k 0.37 and 0.76, 200k 2.8 and 7.2).
+//
+// QBC_TREE_MIN_PAIRS overrides all of it for tests.
 static int64_t min_pairs(const Handle &h, bool rerun) {
   const char *e = std::getenv("QBC_TREE_MIN_PAIRS");
   if (e && *e) return std::strtoll(e, nullptr, 10);
-  if (h.host.kind == IndexKind::CSR) return 0;  // (one source of 100 vertices 0.146 against 0.170 ms)
+  const int32_t n = h.host.n;
+  if (h.host.kind == IndexKind::CSR) return 0;
   if (h.host.kind == IndexKind::H2H) return rerun ? 1000 : 1 << 20;
-  return rerun ? std::max<int64_t>(0, 3600000 - 68 * (int64_t)h.host.n) : 2 << 20;
+  struct Knot {
+    int32_t n;
+    int64_t pairs;
+  };
+  static constexpr Knot wait[] = {{0, 1300000}, {4000, 2900000}, {8000, 2900000}, {28000, 1400000}, {60000, 1300000}, {72000, 500000},
+                                  {90000, 0}, {180000, 0},    {200000, 360000}};
+  static constexpr Knot enqueue[] = {{0, 1600000}, {4000, 3200000}, {8000, 3200000}, {21000, 2 << 20}};
+  auto at = [n](const Knot *k, int count) {
+    int i = 1;
+    while (i < count && k[i].n <= n) i++;
+    if (i == count) return k[count - 1].pairs;
+    return k[i - 1].pairs + (k[i].pairs - k[i - 1].pairs) * (n - k[i - 1].n) / (k[i].n - k[i - 1].n);
+  };
+  return rerun ? at(wait, 9) : at(enqueue, 4);
 }
 
 bool plan_open(const Handle &h, const DeviceState *d) {

@@ -162,3 +162,29 @@ def test_autotune_on_a_short_list_keeps_the_plan_for_longer_ones(tmp_path):
     idx.autotune(np.arange(0, n, 3, dtype=np.int32))  # long enough for the tree: it wins
     t = idx.get_tuning()
     assert t["keep_plan"] == t["label_warps"] == t["split"] == t["dep_form"] == 0
+
+
+@pytest.mark.parametrize("kind,n,shortcuts,ns,waits,plan", [
+    # below and above the rule's line where a call waits, and where it only enqueues
+    (Q.QBC_INDEX_MHL, 2000, 0.0, 800, True, False), (Q.QBC_INDEX_MHL, 2000, 0.0, 1500, True, True),
+    (Q.QBC_INDEX_MHL, 6000, 0.0, 416, True, False), (Q.QBC_INDEX_MHL, 6000, 0.0, 600, True, True),
+    (Q.QBC_INDEX_MHL, 45000, 0.0, 20, True, False), (Q.QBC_INDEX_MHL, 45000, 0.0, 40, True, True),
+    (Q.QBC_INDEX_MHL, 90000, 0.0, 1, True, True),
+    (Q.QBC_INDEX_MHL, 6000, 0.0, 333, False, False), (Q.QBC_INDEX_MHL, 6000, 0.0, 600, False, True),
+    (Q.QBC_INDEX_MHL, 45000, 0.0, 40, False, False), (Q.QBC_INDEX_MHL, 45000, 0.0, 60, False, True),
+    (Q.QBC_INDEX_CSR, 100, 0.02, 1, True, True), (Q.QBC_INDEX_CSR, 100, 0.02, 1, False, True)])
+def test_route_by_size(kind, n, shortcuts, ns, waits, plan, monkeypatch):
+    n, u, v, w = grid_lines(n, seed=4, shortcut_frac=shortcuts)
+    g = Q.Graph(device=0)
+    g.ReadLines(n, u, v, w)
+    idx = g.build_index(kind, on_device=True)
+    srcs = np.random.default_rng(ns).choice(n, ns, replace=False).astype(np.int32)
+    call = (lambda: idx.bc_sources(srcs)) if waits else (lambda: _device_call(idx, n, srcs))
+    took, got = _launches(idx, call), call()
+    monkeypatch.setenv("QBC_TREE_MIN_PAIRS", "0")
+    with_plan, other = _launches(idx, call), call()
+    monkeypatch.setenv("QBC_TREE_MIN_PAIRS", str(1 << 50))
+    without, want = _launches(idx, call), call()
+    assert with_plan != without
+    assert took == (with_plan if plan else without)
+    assert rel_err(got, want) <= BC_RTOL and rel_err(other, want) <= BC_RTOL
