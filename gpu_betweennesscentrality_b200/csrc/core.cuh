@@ -20,9 +20,9 @@
 // unpacking as they are.
 #pragma once
 
-// Degree up to 3, 4, 5, 6: 42, 30, 24, 20 % of the vertices stay, with 4.8 to 8 arcs each; 200k
-// vertices, 4,096 sources 107, 76, 74, 78 ms, 5,003 vertices, all sources 3.07, 2.69, 2.87, 3.19 ms
-// (both with an earlier form of the sweep).
+// Degree up to 3, 4, 5, 6: 42, 30, 24, 20 % of the vertices stay, with 4.8 to 8 arcs each; 5,003
+// vertices, all sources 2.23, 1.95, 2.05, 2.21 ms, 200k, 4,096 sources 64.4, 52.0, 53.6, 57.0 ms, 1M, 2,048
+// sources 314, 166, 159, 167 ms.
 constexpr int kCoreDegree = 4;
 constexpr int kCoreCrowd = 64;  // no vertex next to a longer list is eliminated: it would be searched each time
 constexpr int kCoreSort = 1024;                         // frontiers from here on are visited in vertex order,

@@ -33,10 +33,11 @@
 //
 // Counts are held in 32 bits as in the label rows.  Those wrap where the true count passes 2^31, and
 // BC is then defined by the wrapped values; here a product that reaches 2^31 sets the wrap word, the
-// kernels leave their results unused, and the call is answered by the label kernels.
+// kernels leave their results unused, and the call is answered by the label kernels, as are all calls
+// after it.  (A sum over entries that a shorter one beats later may set it, too.)
 //
 // All 50,175 sources of the 50k grid: 239.8 ms by the label kernels (label scan 142, dependency pass
-// 77, sorting and gaps), 38.1 ms so; 1,024 sources of 500k 150.8 and 22.1 ms, 6,083 of 6k 3.33 and 1.16.
+// 77, sorting and gaps), 37.1 ms so; 1,024 sources of 500k 150.8 and 22.1 ms, 6,083 of 6k 3.33 and 1.15.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -1344,7 +1345,7 @@ __global__ void __launch_bounds__(kBottomWarps * 32) k_bottom(TreeArgs a, int fi
       } while (pe < (uint32_t)v.y);
       e = lds128(vn.x);
       const bool leaf = v.w & kLeaf;
-      if (leaf && !special) {
+      if (leaf && !special) {  // (its entries are arcs, one path each: one entry's count needs no check)
         const unsigned x0 = m1[0] & mask;  // one entry for the lane's two sources, and for all lanes?
         const bool one = ((m1[0] ^ m2[0]) == mask) & ((m1[1] ^ m2[1]) == mask) & ((m1[1] & mask) == x0);
         int all = 0;
@@ -2277,7 +2278,7 @@ static size_t group_bytes(const TreePlan &p) {
 constexpr int64_t kWideCtas = 148 * 12;
 
 // Groups of sources that the per-source scratch holds, at most kMaxGroups.
-constexpr int kMaxGroups = 1024;  // (all sources of 50k in passes of 96, 192, 264 groups: 44.3, 39.1, 37.2 ms)
+constexpr int kMaxGroups = 1024;  // (all sources of 50k in passes of 96 and 192 groups: 19 % and 5 % slower than of 264)
 static int groups_fit(const DeviceState *d) {
   const size_t room = (size_t)d->chunk * d->n_pad * sizeof(int4);
   size_t fit = std::min<size_t>(kMaxGroups, room / group_bytes(*d->tree));
@@ -2403,8 +2404,8 @@ static void launch_bottom(const TreeArgs &a, bool early, int first, int end, int
 static void launch_bottoms(DeviceState *d, const TreeArgs &a, cudaStream_t st) {
   const TreePlan &p = *d->tree;
   if (a.ng > 4) {
-    // A launch runs into the tail of the one before it: all sources of 2k, 6k, 50k vertices 0.444 -> 0.394,
-    // 1.199 -> 1.125, 37.2 -> 36.4 ms, of a 5k core graph 2.00 -> 1.94.  A large core has so many bottoms that
+    // A launch runs into the tail of the one before it: all sources of 2k vertices 0.444 -> 0.394 ms, 6k 6 %
+    // less, 50k 2 %, a 5k core graph 3 %.  A large core has so many bottoms that
     // there is no tail to speak of, and the classes are better kept apart (200k + 2 %: 52.6 against 52.2 ms).
     const bool overlap = p.core.nc < kCoreSmall;
     for (const TreePlan::BotClass &c : p.bot_class) {

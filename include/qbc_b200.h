@@ -149,8 +149,14 @@ int qbc_index_export(const qbc_index *idx, int32_t *vid_of, int32_t *depth, int3
  * With [0], [2], [5]-[9], [12] and [13] all 0, or [14] 1, BC of many (source, vertex) pairs runs over the
  * elimination tree (label indexes built here, not loaded from a file) or over the core graph (CSR
  * index; [10] and [11] apply, [11] = 0 chooses by the core's size) instead of the label, sweep and
- * dependency kernels; any of those fields set asks for the latter.  A path count past 2^31 does, too,
- * from the call that meets it on. */
+ * dependency kernels; any of those fields set asks for the latter.  So does, without notice:
+ *  - a label index whose longest label (half the longest distance or more) reaches 2^(30 - b), b the
+ *    bits of the tree width + 2, at least 6: 4.19M at width 196 (50k grid), 524k at 1,057 (1M grid);
+ *    choose the unit of the weights accordingly;
+ *  - a tree of more than about 10,000 levels, and a core of more than three quarters of the graph;
+ *  - a label-free index where a length that its elimination meets passes 1,973,790, and, from the call
+ *    that meets it on, a distance of 33,554,432 or more (likewise a path count past 2^31 on any index).
+ * A label index keeps its separators on the host (16 B per shortcut, 190 MB at 1M vertices). */
 int qbc_index_set_tuning(qbc_index *idx, const int32_t *params, int32_t nparams);
 int qbc_index_get_tuning(const qbc_index *idx, int32_t *params, int32_t nparams);
 
