@@ -2477,26 +2477,44 @@ static void alloc_scratch(Handle &h, DeviceState *d) {
     chunk = std::max(32, (chunk / 32) * 32);
   }
   chunk = std::min<int32_t>(chunk, std::max(32, (ix.n + 31) / 32 * 32));
-  d->chunk = chunk;
   // one buffer: the label scan and dependency pass of consecutive chunks run in order on one stream
-  for (int b = 0; b < 1; b++) {
-    d->rec[b] = dmalloc<int4>(d, (size_t)chunk * d->n_pad);
-    d->hop[b] = dmalloc<int32_t>(d, (size_t)chunk * d->n_pad);
-    d->order[b] = dmalloc<int32_t>(d, (size_t)chunk * d->n_pad);
-    d->lcnt[b] = dmalloc<int32_t>(d, (size_t)chunk * 2 * (d->n_pad + 2));
-    d->src[b] = dmalloc<int32_t>(d, (size_t)chunk);
-    d->maxhop[b] = dmalloc<int32_t>(d, (size_t)chunk);
-    d->src_rows[b] = dmalloc<int32_t>(d, (size_t)chunk * 2 * d->hmax_pad);
+  try {
+    for (int b = 0; b < 1; b++) {
+      d->rec[b] = dmalloc<int4>(d, (size_t)chunk * d->n_pad);
+      d->hop[b] = dmalloc<int32_t>(d, (size_t)chunk * d->n_pad);
+      d->order[b] = dmalloc<int32_t>(d, (size_t)chunk * d->n_pad);
+      d->lcnt[b] = dmalloc<int32_t>(d, (size_t)chunk * 2 * (d->n_pad + 2));
+      d->src[b] = dmalloc<int32_t>(d, (size_t)chunk);
+      d->maxhop[b] = dmalloc<int32_t>(d, (size_t)chunk);
+      d->src_rows[b] = dmalloc<int32_t>(d, (size_t)chunk * 2 * d->hmax_pad);
+    }
+  } catch (...) {
+    d->scratch_bytes = d->bytes - before;
+    free_scratch(d);
+    throw;
   }
+  d->chunk = chunk;
   d->scratch_bytes = d->bytes - before;
 }
 
 void device_set_chunk(Handle &h, int32_t chunk) {
-  DeviceState *d = need_dev(h);
+  DeviceState *d = need_dev(h, false);
   CK(cudaDeviceSynchronize());
+  const int32_t before = d->chunk;
   free_scratch(d);
   h.tuning.chunk = chunk;
-  alloc_scratch(h, d);
+  try {
+    alloc_scratch(h, d);
+  } catch (...) {  // no room for so many: the size it had (else none, and need_dev refuses calls)
+    cudaGetLastError();
+    h.tuning.chunk = before;
+    try {
+      if (before > 0) alloc_scratch(h, d);
+    } catch (...) {
+      cudaGetLastError();
+    }
+    throw;
+  }
 }
 
 // ------------------------------------------------------------------------------- dense elimination
@@ -3453,9 +3471,10 @@ void device_release(Handle &h) {
 int64_t device_bytes(const Handle &h) { return h.dev ? h.dev->bytes : 0; }
 int device_id(const Handle &h) { return h.dev ? h.dev->device : -1; }
 
-DeviceState *need_dev(Handle &h) {
+DeviceState *need_dev(Handle &h, bool scratch) {
   if (!h.dev) throw Error(QBC_EINVAL, "index is not on a device: call qbc_index_upload first");
   if (h.server) throw Error(QBC_EBUSY, "the index is serving requests: close its server first");
+  if (scratch && h.dev->chunk < 1) throw Error(QBC_ENOMEM, "the index has no per-source scratch: set a smaller chunk");
   CK(cudaSetDevice(h.dev->device));
   return h.dev;
 }

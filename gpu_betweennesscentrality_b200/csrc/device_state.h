@@ -180,7 +180,8 @@ void launch_sweep_rows_grid(const Handle &h, DeviceState *d, int4 *rec, int32_t 
 void launch_tid_to_vid(DeviceState *d, const double *in_tid, double *out_vid, int accumulate, cudaStream_t st);
 // tids of cnt vids (sets ERR_BAD_SOURCE for ids out of range)
 void launch_vid_to_tid(DeviceState *d, const int32_t *vids, int32_t *tids, int32_t cnt, cudaStream_t st);
-DeviceState *need_dev(Handle &h);
+// scratch: the caller needs the per-source buffers
+DeviceState *need_dev(Handle &h, bool scratch = true);
 // frees the captured sweep graphs (they hold scratch pointers; called whenever scratch changes)
 void sweep_cache_free(DeviceState *d);
 // reads and clears the device error word; throws QBC_EDEVICE when a kernel set it (synchronous).

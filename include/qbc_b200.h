@@ -145,7 +145,8 @@ int qbc_index_export(const qbc_index *idx, int32_t *vid_of, int32_t *depth, int3
  * 64-entry blocks through a ring; 0 = auto: whole rows when they fit with 16 warps),
  * [14]=1: [0], [2], [5]-[9], [12] and [13] configure the label kernels for the calls that are too
  * small for the elimination tree (below) without asking for them in the others; a list of fewer
- * params leaves it 0.  Refused with QBC_EBUSY while the index serves.
+ * params leaves it 0.  Refused with QBC_EBUSY while the index serves; a [3] that does not fit the
+ * device with QBC_ENOMEM, the chunk staying as it was.
  * With [0], [2], [5]-[9], [12] and [13] all 0, or [14] 1, BC of many (source, vertex) pairs runs over the
  * elimination tree (label indexes built here, not loaded from a file) or over the core graph (CSR
  * index; [10] and [11] apply, [11] = 0 chooses by the core's size) instead of the label, sweep and

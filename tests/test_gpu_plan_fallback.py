@@ -8,6 +8,7 @@ import pytest
 import gpu_betweennesscentrality_b200 as Q
 import pyoracle as O
 from conftest import rel_err
+from gpu_betweennesscentrality_b200 import capi
 from util import BC_RTOL, grid_lines, lines_of, unit_grid_lines
 
 pytestmark = pytest.mark.gpu
@@ -188,3 +189,22 @@ def test_route_by_size(kind, n, shortcuts, ns, waits, plan, monkeypatch):
     assert with_plan != without
     assert took == (with_plan if plan else without)
     assert rel_err(got, want) <= BC_RTOL and rel_err(other, want) <= BC_RTOL
+
+
+def test_chunk_that_does_not_fit_leaves_the_scratch():
+    """200,000 slots of 200,000 vertices are 1.4 TB: refused, and the next calls are answered as before"""
+    n, u, v, w = grid_lines(200000, seed=4, shortcut_frac=0.02)
+    g = Q.Graph(device=0)
+    g.ReadLines(n, u, v, w)
+    idx = g.build_index(Q.QBC_INDEX_CSR)
+    srcs = np.arange(0, n, n // 40, dtype=np.int32)
+    want, size = idx.bc_sources(srcs), idx.info()
+    for _ in range(2):
+        with pytest.raises(Q.QbcError) as e:
+            idx.set_tuning(chunk=200000)
+        assert e.value.code == capi.QBC_ENOMEM
+        assert np.array_equal(idx.info(), size)  # the same device bytes
+        assert rel_err(idx.bc_sources(srcs), want) <= BC_RTOL
+        assert rel_err(idx.bc_query_batch([srcs], srcs)[0], want[srcs]) <= BC_RTOL
+    idx.set_tuning(chunk=64)
+    assert rel_err(idx.bc_sources(srcs), want) <= BC_RTOL
